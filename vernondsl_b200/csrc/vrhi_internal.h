@@ -194,6 +194,30 @@ inline int element_count(uint64_t rows, uint64_t cols, const char *name, uint64_
   return VRHI_OK;
 }
 
+// Programmatic dependent launch of a kernel that finishes what the kernel before it on the stream began
+// (adds up its partial sums).  The blocks of `kern` become resident as soon as every block of the kernel before it
+// has executed pdl_release() or ended, so its launch latency runs under that kernel; it must execute
+// pdl_wait() before it reads anything, which returns when the kernel before it has completed.  Whatever is
+// launched next in the ordinary way finds both finished.
+template <class Kern, class... Args>
+cudaError_t launch_dependent(Kern kern, dim3 grid, unsigned block, size_t dyn, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = dyn;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 inline int post_launch(vrhi_stream_t *st, const char *what, int kernels = 1) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(VRHI_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
