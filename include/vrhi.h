@@ -353,13 +353,17 @@ typedef struct vrhi_tape_params {
   uint32_t flags; /* VRHI_TAPE_FLAG_* */
   uint32_t colsum_mask; /* bit k: output k is not stored; its column sums are: the argument is a [cols] array.
                            Needs the compiled path (VRHI_ERR_UNSUPPORTED otherwise). Deterministic: fixed order. */
+  uint32_t total_mask;  /* read only with VRHI_TAPE_FLAG_TOTALS.  Bit k: output k is one value, the sum of all its
+                           elements; bit 8+k (with bit k): their mean.  Needs the compiled path. Deterministic. */
 } vrhi_tape_params;
 /* A tape normally runs as a kernel compiled for it at first use (NVRTC, cached; values in
  * registers, HBM-bound).  This flag, or VRHI_TAPE_JIT=0 in the environment, selects the
- * interpreting kernel instead, which is also what runs where NVRTC is not installed, for column
- * counts that are not a multiple of 4 and for unaligned arrays.  Both give the same bits. */
+ * interpreting kernel instead, which is also what runs where NVRTC is not installed, for unaligned
+ * arrays and for a few hundred elements in rows of no multiple of 4.  Both give the same bits. */
 #define VRHI_TAPE_FLAG_INTERPRET 1u
-/* Tapes compiled so far in this process, launches of compiled tapes, the version of the run-time
+#define VRHI_TAPE_FLAG_TOTALS 2u
+/* Tapes compiled so far in this process, launches of compiled tapes (those over rows of a multiple of 4
+ * elements; the forms for other row lengths are not counted), the version of the run-time
  * compiler in use (major*1000 + minor*10; 0 before the first tape, or when there is none) and the
  * CUDA version the library was built with, counted the same way.  When the two versions are equal
  * the compiled and the interpreting kernel give the same bits; with another compiler version the

@@ -738,9 +738,9 @@ struct Planner {
         }
       }
       // A full-size elementwise value whose only reader is a column sum is never written: the map kernel
-      // that computes it adds it up column by column (compiled tapes only, columns a multiple of 4).
+      // that computes it adds it up column by column (compiled tapes only).
       folded.clear(); folded_nodes.clear(); folded_mid.clear();
-      if (g->cols % 4 == 0 && tape_jit_available()) {
+      if (tape_jit_available()) {
         // readers that need the value in memory: reductions and softmax (elementwise readers recompute it
         // inside their own kernel from the leaves)
         std::vector<int> readers(N, 0);

@@ -453,6 +453,7 @@ static int plan_tape(const vrhi_tape_params &q, TapeDev *T, int max_slots) {
 int launch_map_tape(vrhi_stream_t *st, const ArgView *args, int n_args, const void *params, size_t params_size) {
   vrhi_tape_params q;
   VRHI_TRY(read_params(params, params_size, &q));
+  if (!(q.flags & VRHI_TAPE_FLAG_TOTALS)) q.total_mask = 0;
   if (q.n_inputs > VRHI_TAPE_MAX_INPUTS || q.n_outputs == 0 || q.n_outputs > VRHI_TAPE_MAX_OUTPUTS || q.n_instr > VRHI_TAPE_MAX_INSTR)
     return fail(VRHI_ERR_INVALID, "map_tape: %u inputs / %u outputs / %u instructions outside the limits (%d / 1..%d / %d)", q.n_inputs, q.n_outputs, q.n_instr, VRHI_TAPE_MAX_INPUTS, VRHI_TAPE_MAX_OUTPUTS, VRHI_TAPE_MAX_INSTR);
   if (n_args != (int)(q.n_inputs + q.n_outputs)) return fail(VRHI_ERR_INVALID, "map_tape: %d arguments passed, tape declares %u inputs + %u outputs", n_args, q.n_inputs, q.n_outputs);
@@ -461,6 +462,7 @@ int launch_map_tape(vrhi_stream_t *st, const ArgView *args, int n_args, const vo
   if (n == 0) return VRHI_OK;
   if ((q.row_vector_mask & q.col_vector_mask) | (q.row_vector_mask & q.scalar_mask) | (q.col_vector_mask & q.scalar_mask))
     return fail(VRHI_ERR_INVALID, "map_tape: an input is marked with more than one broadcast shape");
+  if (q.colsum_mask & q.total_mask) return fail(VRHI_ERR_INVALID, "map_tape: an output is marked both as column sums and as one sum");
   VRHI_TRY(validate_tape(q));
   TapeDev T{};
   T.n_inputs = q.n_inputs; T.n_outputs = q.n_outputs;
@@ -473,7 +475,7 @@ int launch_map_tape(vrhi_stream_t *st, const ArgView *args, int n_args, const vo
   }
   for (uint32_t k = 0; k < q.n_outputs; ++k) {
     const ArgView &o = args[q.n_inputs + k];
-    const uint64_t out_bytes = ((q.colsum_mask >> k) & 1u) ? q.cols * 4 : n * 4;
+    const uint64_t out_bytes = ((q.colsum_mask >> k) & 1u) ? q.cols * 4 : tape_total(q, k) ? 4 : n * 4;
     if (o.bytes < out_bytes) return fail(VRHI_ERR_SIZE, "map_tape: output %u holds %llu bytes, %llu needed", k, (unsigned long long)o.bytes, (unsigned long long)out_bytes);
     if (!writable(o)) return fail(VRHI_ERR_INVALID, "map_tape: output %u is read-only (class %s)", k, vrhi_arg_class_name(o.buf_cls));
     T.out[k] = (float *)o.ptr;
@@ -484,7 +486,7 @@ int launch_map_tape(vrhi_stream_t *st, const ArgView *args, int n_args, const vo
     const int rc = tape_jit_launch(st, q, T.in, T.out);
     if (rc == VRHI_OK) return post_launch(st, "map_tape (compiled)");
     if (rc != 1) return rc;
-    if (q.colsum_mask) return fail(VRHI_ERR_UNSUPPORTED, "map_tape: column-summed outputs need the compiled path (run-time compiler present, columns a multiple of 4, 16-byte aligned arrays)");
+    if (q.colsum_mask | q.total_mask) return fail(VRHI_ERR_UNSUPPORTED, "map_tape: summed outputs need the compiled path (run-time compiler present, 16-byte aligned arrays)");
   }
   const int slot_capacity = kTapeSlotBytes / (kTapeThreads * (int)sizeof(float4));  // 24 slots of one group
   VRHI_TRY(plan_tape(q, &T, slot_capacity));

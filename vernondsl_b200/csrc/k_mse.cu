@@ -19,8 +19,6 @@
 
 namespace vrhi {
 
-int col_finalize(vrhi_stream_t *st, const float *partial, float *out, uint32_t groups, uint64_t cols, float scale);
-
 struct TanhPair {
   float y;      // tanh(u)
   float sech2;  // 1 - tanh(u)^2
@@ -159,21 +157,6 @@ __global__ void __launch_bounds__(256) mse_fwd_kernel(const float *__restrict__ 
   if (threadIdx.x == 0) loss_partial[(uint64_t)blockIdx.y * gridDim.x + blockIdx.x] = bl;
 }
 
-// Adds the per-block partial sums in index order, in binary64, and scales.
-__global__ void __launch_bounds__(256) loss_finalize_kernel(const float *__restrict__ partial, uint32_t n, double scale,
-                                                            float *__restrict__ out) {
-  __shared__ double sm[256];
-  double s = 0.0;
-  for (uint32_t k = threadIdx.x; k < n; k += 256) s += (double)partial[k];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = (float)(sm[0] * scale);
-}
-
 struct MsePlan {
   uint64_t rows, cols;
   double denom;
@@ -224,8 +207,10 @@ int launch_mse_tanh_fwd(vrhi_stream_t *st, const ArgView *args, int n_args, cons
   if (pl.vec) mse_fwd_kernel<true><<<grid, 256, 0, st->s>>>(W, X, B, T, (float *)payload, pl.rows, pl.cols);
   else mse_fwd_kernel<false><<<grid, 256, 0, st->s>>>(W, X, B, T, (float *)payload, pl.rows, pl.cols);
   VRHI_TRY(post_launch(st, "mse_tanh_fwd"));
-  loss_finalize_kernel<<<1, 256, 0, st->s>>>((const float *)payload, (uint32_t)n_part, 1.0 / pl.denom, (float *)args[4].ptr);
-  return post_launch(st, "loss_finalize");
+  FinishJobs jobs{};
+  add_finish_job(&jobs, (const float *)payload, (float *)args[4].ptr, (uint32_t)n_part, 1, 1.0 / pl.denom);
+  VRHI_CUDA(finish_partials(st->s, jobs));
+  return post_launch(st, "mse_tanh_fwd (second stage)");
 }
 
 int launch_mse_tanh_bwd(vrhi_stream_t *st, const ArgView *args, int n_args, const void *params, size_t params_size) {
@@ -250,12 +235,11 @@ int launch_mse_tanh_bwd(vrhi_stream_t *st, const ArgView *args, int n_args, cons
   if (pl.vec) mse_bwd_kernel<true><<<grid, 256, 0, st->s>>>(W, X, B, T, (float *)args[4].ptr, (float *)args[5].ptr, db_partial, loss_partial, pl.rows, pl.cols, inv);
   else mse_bwd_kernel<false><<<grid, 256, 0, st->s>>>(W, X, B, T, (float *)args[4].ptr, (float *)args[5].ptr, db_partial, loss_partial, pl.rows, pl.cols, inv);
   VRHI_TRY(post_launch(st, "mse_tanh_bwd"));
-  VRHI_TRY(col_finalize(st, db_partial, (float *)args[6].ptr, pl.gy, pl.cols, 1.0f));
-  if (n_args == 8) {
-    loss_finalize_kernel<<<1, 256, 0, st->s>>>((const float *)loss_partial, (uint32_t)n_part, 1.0 / pl.denom, (float *)args[7].ptr);
-    VRHI_TRY(post_launch(st, "loss_finalize"));
-  }
-  return VRHI_OK;
+  FinishJobs jobs{};
+  add_finish_job(&jobs, db_partial, (float *)args[6].ptr, pl.gy, pl.cols, 1.0);
+  if (n_args == 8) add_finish_job(&jobs, loss_partial, (float *)args[7].ptr, (uint32_t)n_part, 1, 1.0 / pl.denom);
+  VRHI_CUDA(finish_partials(st->s, jobs));
+  return post_launch(st, "mse_tanh_bwd (second stage)");
 }
 
 }  // namespace vrhi

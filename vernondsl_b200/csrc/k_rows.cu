@@ -398,28 +398,31 @@ __global__ void __launch_bounds__(256, kColBlocksPerSm<VEC>) col_partial_kernel(
   if (active && sub == 0) static_cast<V *>(partial_raw)[(uint64_t)blockIdx.y * groups + g] = acc;
 }
 
-// Stage 2: a block of 1024 threads owns min(cols, 32) adjacent columns; its threads take the partial rows in
-// turn (coalesced, four independent loads each) and are combined in a tree.  It is latency-bound, so the
-// rows are spread over many threads (with eight warps per 32 columns, 1000 partial rows took 30 us) and it is
-// launched as a dependent of stage 1.
-__global__ void __launch_bounds__(1024) col_finalize_kernel(const float *__restrict__ partial, float *__restrict__ out, uint32_t groups,
-                                                            uint64_t cols, uint32_t W, float scale) {
-  __shared__ float red[1024];
-  const uint32_t R = 1024u / W;
+// Stage 2: a block of 1024 threads owns min(cols, 32) adjacent columns of one job; its threads take the partial rows in
+// turn (coalesced, four independent loads each) and are combined in a tree, in binary64.  It is latency-bound, so the
+// rows are spread over many threads (with eight warps per 32 columns, 1000 partial rows took 30 us), every sum that a
+// kernel left behind is finished by one launch, and that launch is a dependent of stage 1.
+__global__ void __launch_bounds__(1024) finish_partials_kernel(const __grid_constant__ FinishJobs jobs) {
+  __shared__ double red[1024];
+  int j = 0;
+  while (j + 1 < jobs.n && blockIdx.x >= jobs.job[j].last_block) ++j;
+  const FinishJobs::Job &J = jobs.job[j];
+  const uint32_t block = blockIdx.x - (j ? jobs.job[j - 1].last_block : 0u), W = J.W, R = 1024u / W, groups = J.groups;
+  const uint64_t cols = J.cols;
   const uint32_t sub = threadIdx.x / W, w = threadIdx.x - sub * W;
-  const uint64_t c = (uint64_t)blockIdx.x * W + w;
+  const uint64_t c = (uint64_t)block * W + w;
   const bool active = sub < R && c < cols;
   pdl_wait();
-  float s = 0.f;
+  double s = 0.0;
   if (active) {
     uint32_t g = sub;
-    const float *p = partial + (uint64_t)sub * cols + c;
+    const float *p = J.partial + (uint64_t)sub * cols + c;
     const uint64_t pstep = (uint64_t)R * cols;
     for (; g + 3 * R < groups; g += 4 * R, p += 4 * pstep) {
-      const float a = p[0], b = p[pstep], d = p[2 * pstep], e = p[3 * pstep];
+      const double a = p[0], b = p[pstep], d = p[2 * pstep], e = p[3 * pstep];
       s += (a + b) + (d + e);
     }
-    for (; g < groups; g += R, p += pstep) s += *p;
+    for (; g < groups; g += R, p += pstep) s += (double)*p;
   }
   red[threadIdx.x] = s;
   for (uint32_t n = R < groups ? R : groups; n > 1;) {
@@ -431,18 +434,19 @@ __global__ void __launch_bounds__(1024) col_finalize_kernel(const float *__restr
     }
     n = half;
   }
-  if (active && sub == 0) out[c] = s * scale;
+  if (active && sub == 0) J.out[c] = (float)(s * J.scale);
 }
 
-static cudaError_t launch_col_finalize(cudaStream_t s, const float *partial, float *out, uint32_t groups, uint64_t cols, float scale) {
-  const uint32_t W = (uint32_t)(cols < 32 ? cols : 32);
-  return launch_dependent(col_finalize_kernel, dim3((unsigned)((cols + W - 1) / W)), 1024, 0, s, partial, out, groups, cols, W, scale);
+void add_finish_job(FinishJobs *jobs, const float *partial, float *out, uint32_t groups, uint64_t cols, double scale) {
+  FinishJobs::Job &J = jobs->job[jobs->n];
+  J.partial = partial; J.out = out; J.scale = scale; J.cols = cols; J.groups = groups;
+  J.W = (uint32_t)(cols < 32 ? cols : 32);
+  J.last_block = (uint32_t)((cols + J.W - 1) / J.W) + (jobs->n ? jobs->job[jobs->n - 1].last_block : 0u);
+  ++jobs->n;
 }
 
-// Shared with the backward kernel and the compiled tapes: sums `groups` partial rows of `cols` floats into out.
-int col_finalize(vrhi_stream_t *st, const float *partial, float *out, uint32_t groups, uint64_t cols, float scale) {
-  VRHI_CUDA(launch_col_finalize(st->s, partial, out, groups, cols, scale));
-  return post_launch(st, "col_finalize");
+cudaError_t finish_partials(cudaStream_t s, const FinishJobs &jobs) {
+  return launch_dependent(finish_partials_kernel, dim3(jobs.job[jobs.n - 1].last_block), 1024, 0, s, jobs);
 }
 
 // Tile and grid of stage 1.  Tiles of at most 64 float4 (1 KiB of a row) or 128 columns: several rows per block even
@@ -499,7 +503,11 @@ int launch_col_sum(vrhi_stream_t *st, const ArgView *args, int n_args, const voi
   }
   VRHI_CUDA(launch_col_partial(st->s, p, (const float *)args[0].ptr, dst, q.rows));
   VRHI_TRY(post_launch(st, "col_sum"));
-  return p.gy > 1 ? col_finalize(st, dst, out, p.gy, q.cols, 1.0f) : VRHI_OK;
+  if (p.gy == 1) return VRHI_OK;
+  FinishJobs jobs{};
+  add_finish_job(&jobs, dst, out, p.gy, q.cols, 1.0);
+  VRHI_CUDA(finish_partials(st->s, jobs));
+  return post_launch(st, "col_sum (second stage)");
 }
 
 }  // namespace vrhi
@@ -582,7 +590,11 @@ extern "C" int vrhi_col_sum_static_scratch(const float *in_device, float *out_de
   const bool direct = p.gy == 1 && (!p.vec || reinterpret_cast<uintptr_t>(out_device) % 16 == 0);
   cudaError_t e = launch_col_partial(s, p, in_device, direct ? out_device : partials, rows);
   if (e != cudaSuccess) return fail(VRHI_ERR_CUDA, "launch of col_sum_static_scratch (partials) failed: %s", cudaGetErrorString(e));
-  if (!direct) e = launch_col_finalize(s, partials, out_device, p.gy, cols, 1.0f);
+  if (!direct) {
+    FinishJobs jobs{};
+    add_finish_job(&jobs, partials, out_device, p.gy, cols, 1.0);
+    e = finish_partials(s, jobs);
+  }
   if (e != cudaSuccess) return fail(VRHI_ERR_CUDA, "launch of col_sum_static_scratch (finalize) failed: %s", cudaGetErrorString(e));
   return VRHI_OK;
 }

@@ -68,7 +68,6 @@ bool g_loaded = false;
 uint64_t g_compiled = 0, g_launches = 0;
 struct Compiled {
   CUfunction fn;
-  bool flat;     // no row or column vectors: the kernel indexes the data as one long array
   int resident;  // blocks of 256 threads that fit on one SM at a time
 };
 std::unordered_map<std::string, Compiled> g_cache;  // key: device ordinal + the tape's description
@@ -168,14 +167,33 @@ std::string expression(const vrhi_tape_instr &I) {
   }
 }
 
-// The kernel: 256 threads, each owning one float4 column group; blockIdx.y strides over rows, `unroll`
-// rows per trip with the loads of all of them issued before any is used.  Row vectors are
-// loaded once per thread, column vectors once per row, scalars once per thread.  Without row or
-// column vectors the data is one long array (`flat`): the host picks a convenient row length.
-std::string generate(const vrhi_tape_params &q, bool *flat_out, int unroll = 2) {
+// How a generated kernel walks its arrays.  256 threads per block in every form.
+//   FLAT    no row or column vectors, no column sums: one long array of float4s, grid-stride, whatever the row
+//           length; the up to three elements behind the last float4 are done one by one by the first block.
+//   VECTOR  rows of float4 groups (the row length is a multiple of 4).
+//   SCALAR  rows of single elements (any row length; rows then start at any 4-byte boundary).
+// VECTOR and SCALAR: a block owns a tile of W adjacent groups and takes R = 256 / W rows at a time, thread t the group
+// t % W of the rows t / W, t / W + R, ...: a narrow array keeps the whole block busy, neighbouring threads read
+// neighbouring addresses, and a row vector is loaded once per thread.  W and R are launch parameters.
+enum Form { FLAT, VECTOR, SCALAR };
+
+Form form_of(const vrhi_tape_params &q) {
+  if ((q.row_vector_mask | q.col_vector_mask | q.colsum_mask) == 0) return FLAT;
+  return q.cols % 4 == 0 ? VECTOR : SCALAR;
+}
+
+// `unroll` groups per thread and trip, the loads of all of them issued before any is used.  Row vectors and scalars are
+// loaded once per thread, column vectors once per row.  An output is stored, or (colsum_mask) added up over the rows
+// in a register, over the R rows of the block in shared memory, and written as one partial row per block row, or
+// (total_mask) added up over everything the block visits and written as one partial value per block.
+std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
   const unsigned NI = q.n_inputs, NO = q.n_outputs, NT = q.n_instr;
-  const bool flat = (q.row_vector_mask | q.col_vector_mask) == 0 && q.colsum_mask == 0;  // column sums need a thread to keep its columns
-  *flat_out = flat;
+  const bool vec = form != SCALAR;
+  const std::vector<std::string> comps = vec ? std::vector<std::string>{".x", ".y", ".z", ".w"} : std::vector<std::string>{""};
+  const std::string V = vec ? "float4" : "float", ULL = "unsigned long long";
+  const std::string zero = vec ? "make_float4(0.f, 0.f, 0.f, 0.f)" : "0.f";
+  auto splat = [&](const std::string &e) { return vec ? "make_float4(" + e + ", " + e + ", " + e + ", " + e + ")" : e; };
+  auto str = [](unsigned k) { return std::to_string(k); };
   std::vector<bool> used(NI + NT, false);
   for (unsigned t = 0; t < NT; ++t) {
     const int ar = tape_arity(q.instr[t].op);
@@ -184,79 +202,123 @@ std::string generate(const vrhi_tape_params &q, bool *flat_out, int unroll = 2) 
   }
   for (unsigned k = 0; k < NO; ++k) used[q.out_value[k]] = true;
   auto shape = [&](unsigned k) { return ((q.row_vector_mask >> k) & 1u) ? 'r' : ((q.col_vector_mask >> k) & 1u) ? 'c' : ((q.scalar_mask >> k) & 1u) ? 's' : 'f'; };
+  auto colsum = [&](unsigned k) { return ((q.colsum_mask >> k) & 1u) != 0; };
+  auto total = [&](unsigned k) { return tape_total(q, k); };
+  bool any_colsum = false, any_total = false;
+  for (unsigned k = 0; k < NO; ++k) { any_colsum = any_colsum || colsum(k); any_total = any_total || total(k); }
 
   std::string s = kMathSource;
   s += "\n__device__ __forceinline__ void tape_body(";
   for (unsigned k = 0; k < NI; ++k) s += "const float " + v(k) + ", ";
-  for (unsigned k = 0; k < NO; ++k) s += "float &r" + std::to_string(k) + (k + 1 < NO ? ", " : "");
+  for (unsigned k = 0; k < NO; ++k) s += "float &r" + str(k) + (k + 1 < NO ? ", " : "");
   s += ") {\n";
   for (unsigned t = 0; t < NT; ++t) s += "  const float " + v(NI + t) + " = " + expression(q.instr[t]) + ";\n";
-  for (unsigned k = 0; k < NO; ++k) s += "  r" + std::to_string(k) + " = " + v(q.out_value[k]) + ";\n";
+  for (unsigned k = 0; k < NO; ++k) s += "  r" + str(k) + " = " + v(q.out_value[k]) + ";\n";
   s += "}\n\nextern \"C\" __global__ void __launch_bounds__(256) vrhi_tape_kernel(";
-  for (unsigned k = 0; k < NI; ++k) s += "const float *__restrict__ in" + std::to_string(k) + ", ";
-  for (unsigned k = 0; k < NO; ++k) s += "float *__restrict__ out" + std::to_string(k) + ", ";
-  s += "const unsigned long long n4, const unsigned long long rows, const unsigned long long rows_full, const unsigned int cols4) {\n";
-  s += "  const unsigned int c4 = blockIdx.x * 256u + threadIdx.x;\n  if (c4 >= cols4) return;\n";
+  for (unsigned k = 0; k < NI; ++k) s += "const float *__restrict__ in" + str(k) + ", ";
+  for (unsigned k = 0; k < NO; ++k) s += "float *__restrict__ out" + str(k) + ", ";
+  s += "const " + ULL + " rows, const " + ULL + " groups, const unsigned int W, const unsigned int R, const unsigned int tail) {\n";
+  if (any_colsum || any_total) s += "  asm volatile(\"griddepcontrol.launch_dependents;\");  // the kernel that adds the partial sums may be launched\n";
+  if (form == FLAT) {
+    s += "  " + ULL + " i = (" + ULL + ")blockIdx.x * 256u + threadIdx.x;\n  const " + ULL + " step = (" + ULL + ")gridDim.x * 256u;\n";
+  } else {
+    s += "  const unsigned int sub = threadIdx.x / W, w = threadIdx.x - sub * W;\n";
+    s += "  const " + ULL + " g = (" + ULL + ")blockIdx.x * W + w;\n  const bool active = sub < R && g < groups;\n";
+    s += "  " + ULL + " row = (" + ULL + ")blockIdx.y * R + sub;\n  const " + ULL + " step = (" + ULL + ")gridDim.y * R, istep = step * groups;\n";
+    s += "  " + ULL + " i = row * groups + g;\n";
+  }
   for (unsigned k = 0; k < NI; ++k) {
     if (!used[k]) continue;
-    const std::string K = std::to_string(k);
-    if (shape(k) == 'r') s += "  const float4 x" + K + " = __ldg(reinterpret_cast<const float4 *>(in" + K + ") + c4);\n";
-    if (shape(k) == 's') s += "  const float s" + K + " = __ldg(in" + K + ");\n  const float4 x" + K + " = make_float4(s" + K + ", s" + K + ", s" + K + ", s" + K + ");\n";
+    const std::string K = str(k);
+    if (shape(k) == 'r') s += "  const " + V + " x" + K + " = active ? __ldg(reinterpret_cast<const " + V + " *>(in" + K + ") + g) : " + zero + ";\n";
+    if (shape(k) == 's') s += "  const float s" + K + " = __ldg(in" + K + ");\n  const " + V + " x" + K + " = " + splat("s" + K) + ";\n";
   }
-  // loads of one row group, and its arithmetic and stores
+  for (unsigned k = 0; k < NO; ++k)
+    if (colsum(k) || total(k)) s += "  " + V + " acc" + str(k) + " = " + zero + ";\n";
+  // loads of one group, and its arithmetic and stores
   auto loads = [&](const std::string &G, const std::string &idx, const std::string &row) {
     std::string t;
     for (unsigned k = 0; k < NI; ++k) {
       if (!used[k]) continue;
-      const std::string K = std::to_string(k), name = "x" + K + "_" + G;
-      if (shape(k) == 'f') t += "      const float4 " + name + " = __ldcs(reinterpret_cast<const float4 *>(in" + K + ") + " + idx + ");\n";
-      if (shape(k) == 'c') t += "      const float c" + K + "_" + G + " = __ldg(in" + K + " + " + row + ");\n      const float4 " + name + " = make_float4(c" + K + "_" + G + ", c" + K + "_" + G + ", c" + K + "_" + G + ", c" + K + "_" + G + ");\n";
+      const std::string K = str(k), name = "x" + K + "_" + G;
+      if (shape(k) == 'f') t += "      const " + V + " " + name + " = __ldcs(reinterpret_cast<const " + V + " *>(in" + K + ") + " + idx + ");\n";
+      if (shape(k) == 'c') t += "      const float c" + K + "_" + G + " = __ldg(in" + K + " + " + row + ");\n      const " + V + " " + name + " = " + splat("c" + K + "_" + G) + ";\n";
     }
     return t;
   };
   auto work = [&](const std::string &G, const std::string &idx) {
     std::string t = "      {\n";
-    for (unsigned k = 0; k < NO; ++k) t += "        float4 o" + std::to_string(k) + ";\n";
-    for (const char *comp : {"x", "y", "z", "w"}) {
+    for (unsigned k = 0; k < NO; ++k) t += "        " + V + " o" + str(k) + ";\n";
+    for (const std::string &c : comps) {
       t += "        tape_body(";
       for (unsigned k = 0; k < NI; ++k) {
-        const std::string K = std::to_string(k);
+        const std::string K = str(k);
         if (!used[k]) t += "0.0f, ";
-        else if (shape(k) == 'r' || shape(k) == 's') t += "x" + K + "." + comp + ", ";
-        else t += "x" + K + "_" + G + "." + comp + ", ";
+        else if (shape(k) == 'r' || shape(k) == 's') t += "x" + K + c + ", ";
+        else t += "x" + K + "_" + G + c + ", ";
       }
-      for (unsigned k = 0; k < NO; ++k) t += "o" + std::to_string(k) + "." + comp + (k + 1 < NO ? ", " : "");
+      for (unsigned k = 0; k < NO; ++k) t += "o" + str(k) + c + (k + 1 < NO ? ", " : "");
       t += ");\n";
     }
     for (unsigned k = 0; k < NO; ++k) {
-      const std::string K = std::to_string(k);
-      if ((q.colsum_mask >> k) & 1u)  // rows are visited in a fixed order: the sum does not depend on scheduling
-        t += "        acc" + K + ".x += o" + K + ".x; acc" + K + ".y += o" + K + ".y; acc" + K + ".z += o" + K + ".z; acc" + K + ".w += o" + K + ".w;\n";
-      else
-        t += "        __stcs(reinterpret_cast<float4 *>(out" + K + ") + " + idx + ", o" + K + ");\n";
+      const std::string K = str(k);
+      if (colsum(k) || total(k)) {  // groups are visited in a fixed order: the sum does not depend on scheduling
+        t += "       ";
+        for (const std::string &c : comps) t += " acc" + K + c + " += o" + K + c + ";";
+        t += "\n";
+      } else {
+        t += "        __stcs(reinterpret_cast<" + V + " *>(out" + K + ") + " + idx + ", o" + K + ");\n";
+      }
     }
     return t + "      }\n";
   };
-  for (unsigned k = 0; k < NO; ++k)
-    if ((q.colsum_mask >> k) & 1u) s += "  float4 acc" + std::to_string(k) + " = make_float4(0.f, 0.f, 0.f, 0.f);\n";
-  s += "  unsigned long long row = blockIdx.y;\n";
-  const std::string U = std::to_string(unroll);
-  s += "  for (; row + " + std::to_string(unroll - 1) + "ull * gridDim.y < rows_full; row += " + U + "ull * gridDim.y) {  // " + U + " complete rows per trip: all loads first\n";
-  for (int g = 0; g < unroll; ++g) {
-    const std::string G = std::to_string(g);
-    s += "      const unsigned long long row_" + G + " = row + " + G + "ull * gridDim.y, i" + G + " = row_" + G + " * cols4 + c4;\n";
+  const std::string U = str((unsigned)unroll), last = str((unsigned)unroll - 1);
+  const std::string advance = form == FLAT ? "i += " + U + "ull * step" : "row += " + U + "ull * step, i += " + U + "ull * istep";
+  const std::string pos = form == FLAT ? "i" : "row", most = form == FLAT ? "groups" : "rows", di = form == FLAT ? "step" : "istep";
+  if (form != FLAT) s += "  if (active) {\n";
+  s += "  for (; " + pos + " + " + last + "ull * step < " + most + "; " + advance + ") {  // " + U + " complete groups per trip: all loads first\n";
+  for (int k = 0; k < unroll; ++k) {
+    const std::string G = str((unsigned)k);
+    s += "      const " + ULL + " i" + G + " = i + " + G + "ull * " + di + (form == FLAT ? "" : ", row_" + G + " = row + " + G + "ull * step") + ";\n";
   }
-  for (int g = 0; g < unroll; ++g) s += loads(std::to_string(g), "i" + std::to_string(g), "row_" + std::to_string(g));
-  for (int g = 0; g < unroll; ++g) s += work(std::to_string(g), "i" + std::to_string(g));
+  for (int k = 0; k < unroll; ++k) s += loads(str((unsigned)k), "i" + str((unsigned)k), "row_" + str((unsigned)k));
+  for (int k = 0; k < unroll; ++k) s += work(str((unsigned)k), "i" + str((unsigned)k));
   s += "  }\n";
-  s += "  for (; row < rows; row += gridDim.y) {  // rows left over; the last one may be ragged\n";
-  s += "      const unsigned long long i0 = row * cols4 + c4;\n      if (i0 >= n4) break;\n";
-  s += loads("0", "i0", "row") + work("0", "i0");
+  s += "  for (; " + pos + " < " + most + "; " + (form == FLAT ? "i += step" : "row += step, i += istep") + ") {  // groups left over\n";
+  s += loads("0", "i", "row") + work("0", "i");
   s += "  }\n";
-  // column-summed outputs: this block's partial row, [gridDim.y][cols]; a second kernel adds the partial rows
-  for (unsigned k = 0; k < NO; ++k)
-    if ((q.colsum_mask >> k) & 1u)
-      s += "  reinterpret_cast<float4 *>(out" + std::to_string(k) + ")[(unsigned long long)blockIdx.y * cols4 + c4] = acc" + std::to_string(k) + ";\n";
+  if (form != FLAT) s += "  }\n";
+  if (form == FLAT) {  // the elements behind the last float4
+    s += "  if (blockIdx.x == 0 && threadIdx.x < tail) {\n      const " + ULL + " e = 4ull * groups + threadIdx.x;\n";
+    for (unsigned k = 0; k < NO; ++k) s += "      float o" + str(k) + ";\n";
+    s += "      tape_body(";
+    for (unsigned k = 0; k < NI; ++k) s += !used[k] ? std::string("0.0f, ") : shape(k) == 's' ? "s" + str(k) + ", " : "in" + str(k) + "[e], ";
+    for (unsigned k = 0; k < NO; ++k) s += "o" + str(k) + (k + 1 < NO ? ", " : "");
+    s += ");\n";
+    for (unsigned k = 0; k < NO; ++k) s += total(k) ? "      acc" + str(k) + ".x += o" + str(k) + ";\n" : "      out" + str(k) + "[e] = o" + str(k) + ";\n";
+    s += "  }\n";
+  }
+  // column-summed outputs: a tree over the block's R rows, then this block row's partial row, [gridDim.y][groups]
+  if (any_colsum) s += "  __shared__ " + V + " red[256];\n";
+  for (unsigned k = 0; k < NO; ++k) {
+    if (!colsum(k)) continue;
+    const std::string K = str(k);
+    s += "  if (R > 1) {\n    __syncthreads();\n    red[threadIdx.x] = acc" + K + ";\n    for (unsigned int n = R; n > 1;) {\n      const unsigned int half = (n + 1) >> 1;\n      __syncthreads();\n";
+    s += "      if (active && sub < n - half) {\n        const " + V + " other = red[threadIdx.x + half * W];\n       ";
+    for (const std::string &c : comps) s += " acc" + K + c + " += other" + c + ";";
+    s += "\n        red[threadIdx.x] = acc" + K + ";\n      }\n      n = half;\n    }\n  }\n";
+    s += "  if (active && sub == 0) reinterpret_cast<" + V + " *>(out" + K + ")[(" + ULL + ")blockIdx.y * groups + g] = acc" + K + ";\n";
+  }
+  // summed outputs: one partial value per block
+  if (any_total) s += "  __shared__ float warp_total[8];\n";
+  for (unsigned k = 0; k < NO; ++k) {
+    if (!total(k)) continue;
+    const std::string K = str(k);
+    s += vec ? "  float t" + K + " = (acc" + K + ".x + acc" + K + ".y) + (acc" + K + ".z + acc" + K + ".w);\n" : "  float t" + K + " = acc" + K + ";\n";
+    s += "  for (int o = 16; o > 0; o >>= 1) t" + K + " += __shfl_xor_sync(0xffffffffu, t" + K + ", o);\n";
+    s += "  __syncthreads();\n  if ((threadIdx.x & 31u) == 0) warp_total[threadIdx.x >> 5] = t" + K + ";\n  __syncthreads();\n";
+    s += "  if (threadIdx.x == 0) {\n    float t = warp_total[0];\n    for (int j = 1; j < 8; ++j) t += warp_total[j];\n    out" + K + "[(" + ULL + ")blockIdx.y * gridDim.x + blockIdx.x] = t;\n  }\n";
+  }
   s += "}\n";
   return s;
 }
@@ -300,46 +362,49 @@ int compile(vrhi_device_t *dev, const std::string &src, CUfunction *out) {
 
 }  // namespace
 
-// Returns VRHI_OK when the compiled kernel was launched, 1 when this tape or shape is left to the
-// interpreter (no NVRTC, switched off, columns not a multiple of 4, unaligned pointers), and an
-// error code when compilation or the launch failed.
 // VRHI_TAPE_JIT=0 in the environment selects the interpreting kernel for every tape; read once per process
 static bool jit_enabled() {
   static const bool on = env_int("VRHI_TAPE_JIT", 0, 1, 1) != 0;
   return on;
 }
 
+// Returns VRHI_OK when the compiled kernel was launched, 1 when this tape or shape is left to the
+// interpreter (no NVRTC, switched off, unaligned pointers, a handful of elements), and an error code when
+// compilation or the launch failed.
 int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *const *in, float *const *out) {
   if (q.flags & VRHI_TAPE_FLAG_INTERPRET) return 1;
   if (!jit_enabled()) return 1;
-  if (q.cols % 4 != 0) return 1;
-  for (uint32_t k = 0; k < q.n_inputs; ++k)
-    if (!((q.col_vector_mask >> k) & 1u) && !((q.scalar_mask >> k) & 1u) && ((uintptr_t)in[k] % 16)) return 1;
-  for (uint32_t k = 0; k < q.n_outputs; ++k)
-    if ((uintptr_t)out[k] % 16) return 1;
+  const Form form = form_of(q);
+  const uint64_t n = q.rows * q.cols;
+  // A few hundred elements take the time of a launch either way, and compiling costs a tenth of a second once.
+  if (q.cols % 4 != 0 && n < 256 && !(q.colsum_mask | q.total_mask)) return 1;
+  if (form != SCALAR) {
+    for (uint32_t k = 0; k < q.n_inputs; ++k)
+      if (!((q.col_vector_mask >> k) & 1u) && !((q.scalar_mask >> k) & 1u) && ((uintptr_t)in[k] % 16)) return 1;
+    for (uint32_t k = 0; k < q.n_outputs; ++k)
+      if ((uintptr_t)out[k] % 16) return 1;
+  }
 
   std::lock_guard<std::mutex> lock(g_mu);
   load_once();
   if (!g_nvrtc.ok || !g_driver.ok) return 1;
-  bool flat = false;
-  // About three 16-byte loads in flight per thread and six blocks per SM, all resident at once (one wave):
-  // measured on B200 with the three-input chain, 6.8 TB/s; eight blocks per SM spill into a second, partly
-  // filled wave and two rows per trip then cost 15 %.
+  // FLAT and VECTOR: about three 16-byte loads in flight per thread and six blocks per SM, all resident at once (one
+  // wave): measured on B200 with the three-input chain, 6.8 TB/s; eight blocks per SM spill into a second, partly
+  // filled wave and two rows per trip then cost 15 %.  SCALAR: a load brings a quarter of that, so four rows per trip
+  // (two where an expression reads four arrays and more) and every block that is resident.
   int full_inputs = 0;
   for (uint32_t k = 0; k < q.n_inputs; ++k)
     if (!(((q.row_vector_mask | q.col_vector_mask | q.scalar_mask) >> k) & 1u)) ++full_inputs;
-  int unroll = full_inputs >= 3 ? 1 : full_inputs == 2 ? 2 : 3, blocks_per_sm = 0;  // 0: what is resident at once, at most 6
+  int unroll = form == SCALAR ? (full_inputs >= 4 ? 2 : 4) : full_inputs >= 3 ? 1 : full_inputs == 2 ? 2 : 3;
   static const int env_unroll = env_int("VRHI_TAPE_UNROLL", 1, 8, 0), env_blocks = env_int("VRHI_TAPE_BLOCKS_PER_SM", 1, 32, 0);  // tuning aids
   if (env_unroll) unroll = env_unroll;
-  if (env_blocks) blocks_per_sm = env_blocks;
   // cache key: everything the generated text depends on, as raw bytes (the text itself is only built on a miss)
   std::string key;
   {
-    const uint32_t head[8] = {(uint32_t)st->dev->ordinal, (uint32_t)unroll, q.n_inputs, q.n_outputs, q.n_instr,
-                              q.row_vector_mask, q.col_vector_mask, q.scalar_mask};
+    const uint32_t head[11] = {(uint32_t)st->dev->ordinal, (uint32_t)unroll, (uint32_t)form, q.n_inputs, q.n_outputs, q.n_instr,
+                               q.row_vector_mask, q.col_vector_mask, q.scalar_mask, q.colsum_mask, q.total_mask};
     key.append(reinterpret_cast<const char *>(head), sizeof head);
     key.append(reinterpret_cast<const char *>(q.out_value), sizeof(uint32_t) * q.n_outputs);
-    key.append(reinterpret_cast<const char *>(&q.colsum_mask), sizeof q.colsum_mask);
     for (uint32_t t = 0; t < q.n_instr; ++t) {  // field by field: padding bytes of the struct are not defined
       const vrhi_tape_instr &I = q.instr[t];
       const uint16_t f[4] = {I.op, I.a, I.b, I.c};
@@ -349,7 +414,7 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   }
   auto it = g_cache.find(key);
   if (it == g_cache.end()) {
-    const std::string src = generate(q, &flat, unroll);
+    const std::string src = generate(q, form, unroll);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     VRHI_CUDA(cudaStreamIsCapturing(st->s, &cap));
     if (cap != cudaStreamCaptureStatusNone)
@@ -359,51 +424,75 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
     VRHI_TRY(compile(st->dev, src, &fn));
     int resident = 0;
     if (g_driver.occupancy(&resident, fn, 256, 0) != CUDA_SUCCESS || resident < 1) resident = 4;
-    it = g_cache.emplace(key, Compiled{fn, flat, resident}).first;
+    it = g_cache.emplace(key, Compiled{fn, resident}).first;
     ++g_compiled;
   }
-  const uint64_t n4 = q.rows * q.cols / 4;
-  uint64_t rows = q.rows;
-  uint32_t cols4 = (uint32_t)(q.cols / 4);
-  if (q.cols / 4 > 0xffffffffull) return 1;
-  flat = it->second.flat;
-  if (flat) {  // one long array: rows of 1024 float4 groups, the last one ragged (guarded by n4)
-    cols4 = n4 < 1024 ? (uint32_t)n4 : 1024u;
-    rows = (n4 + cols4 - 1) / cols4;
-  }
-  const unsigned gx = (cols4 + 255u) / 256u;
-  if (blocks_per_sm == 0) blocks_per_sm = it->second.resident < 6 ? it->second.resident : 6;
+  const int most_blocks = form == SCALAR ? 8 : 6;
+  const uint64_t blocks_per_sm = env_blocks ? env_blocks : it->second.resident < most_blocks ? it->second.resident : most_blocks;
   const uint64_t target = (uint64_t)st->dev->prop.multiProcessorCount * blocks_per_sm;
-  uint64_t gy = (target + gx - 1) / gx;
-  const uint64_t row_pairs = (rows + unroll - 1) / unroll;
-  if (gy > row_pairs) gy = row_pairs;
-  if (gy > 65535) gy = 65535;
-  if (gy == 0) gy = 1;
-  void *args[VRHI_TAPE_MAX_INPUTS + VRHI_TAPE_MAX_OUTPUTS + 4];
+  uint64_t rows = q.rows, groups, gx, gy = 1;
+  uint32_t W = 256, R = 1, tail = 0;
+  if (form == FLAT) {
+    groups = n / 4;
+    tail = (uint32_t)(n % 4);
+    gx = (groups + 255) / 256;
+    if (gx > target) gx = target;
+    if (gx == 0) gx = 1;
+  } else {
+    groups = form == VECTOR ? q.cols / 4 : q.cols;
+    // with column sums, tiles of 1 KiB (VECTOR) or half of that: several rows per block, so fewer partial rows
+    const uint64_t most_w = q.colsum_mask ? (form == VECTOR ? 64 : 128) : 256;
+    gx = (groups + most_w - 1) / most_w;
+    if (gx > 0x7fffffffull) return fail(VRHI_ERR_UNSUPPORTED, "map_tape: too many columns");
+    W = (uint32_t)((groups + gx - 1) / gx);
+    R = 256u / W;
+    gy = target / gx;
+    const uint64_t by_rows = (rows + (uint64_t)R * unroll - 1) / ((uint64_t)R * unroll);
+    if (gy > by_rows) gy = by_rows;
+    if (gy > 65535) gy = 65535;
+    if (gy == 0) gy = 1;
+  }
+  void *args[VRHI_TAPE_MAX_INPUTS + VRHI_TAPE_MAX_OUTPUTS + 5];
   const float *in_copy[VRHI_TAPE_MAX_INPUTS];
   float *out_copy[VRHI_TAPE_MAX_OUTPUTS];
-  int n = 0;
-  for (uint32_t k = 0; k < q.n_inputs; ++k) { in_copy[k] = in[k]; args[n++] = &in_copy[k]; }
-  char *scratch = nullptr;
-  if (q.colsum_mask) {
-    const size_t per_output = (size_t)gy * q.cols * sizeof(float);
-    VRHI_TRY(stream_arena(st, per_output * VRHI_TAPE_MAX_OUTPUTS, nullptr, &scratch));
+  int n_args = 0;
+  for (uint32_t k = 0; k < q.n_inputs; ++k) { in_copy[k] = in[k]; args[n_args++] = &in_copy[k]; }
+  FinishJobs jobs{};
+  if (q.colsum_mask | q.total_mask) {
+    const size_t colsum_floats = (size_t)gy * q.cols, total_floats = ((size_t)gx * gy + 3) & ~size_t(3);
+    size_t floats = 0;
+    for (uint32_t k = 0; k < q.n_outputs; ++k) floats += ((q.colsum_mask >> k) & 1u) ? (colsum_floats + 3) & ~size_t(3) : tape_total(q, k) ? total_floats : 0;
+    char *scratch = nullptr;
+    VRHI_TRY(stream_arena(st, floats * sizeof(float), nullptr, &scratch));
+    float *next = reinterpret_cast<float *>(scratch);
+    for (uint32_t k = 0; k < q.n_outputs; ++k) {
+      out_copy[k] = out[k];
+      if ((q.colsum_mask >> k) & 1u) {
+        out_copy[k] = next;
+        next += (colsum_floats + 3) & ~size_t(3);
+        add_finish_job(&jobs, out_copy[k], out[k], (uint32_t)gy, q.cols, 1.0);
+      } else if (tape_total(q, k)) {
+        out_copy[k] = next;
+        next += total_floats;
+        add_finish_job(&jobs, out_copy[k], out[k], (uint32_t)(gx * gy), 1, tape_mean(q, k) ? 1.0 / (double)n : 1.0);
+      }
+    }
+  } else {
+    for (uint32_t k = 0; k < q.n_outputs; ++k) out_copy[k] = out[k];
   }
-  for (uint32_t k = 0; k < q.n_outputs; ++k) {
-    out_copy[k] = ((q.colsum_mask >> k) & 1u) ? reinterpret_cast<float *>(scratch + (size_t)k * gy * q.cols * sizeof(float)) : out[k];
-    args[n++] = &out_copy[k];
-  }
-  uint64_t n4_arg = n4, rows_arg = rows, rows_full = n4 / cols4;  // rows_full: rows that hold all cols4 groups
-  args[n++] = &n4_arg; args[n++] = &rows_arg; args[n++] = &rows_full; args[n++] = &cols4;
-  CUresult cr = g_driver.launch_kernel(it->second.fn, gx, (unsigned)gy, 1, 256, 1, 1, 0, reinterpret_cast<CUstream>(st->s), args, nullptr);
+  for (uint32_t k = 0; k < q.n_outputs; ++k) args[n_args++] = &out_copy[k];
+  args[n_args++] = &rows; args[n_args++] = &groups; args[n_args++] = &W; args[n_args++] = &R; args[n_args++] = &tail;
+  CUresult cr = g_driver.launch_kernel(it->second.fn, (unsigned)gx, (unsigned)gy, 1, 256, 1, 1, 0, reinterpret_cast<CUstream>(st->s), args, nullptr);
   if (cr != CUDA_SUCCESS) {
     const char *msg = "?";
     g_driver.get_error_string(cr, &msg);
     return fail(VRHI_ERR_CUDA, "launch of a compiled tape failed: %s", msg);
   }
-  ++g_launches;
-  for (uint32_t k = 0; k < q.n_outputs; ++k)
-    if ((q.colsum_mask >> k) & 1u) VRHI_TRY(col_finalize(st, out_copy[k], out[k], (uint32_t)gy, q.cols, 1.0f));
+  if (q.cols % 4 == 0) ++g_launches;
+  if (jobs.n) {
+    st->launches += 1;  // the tape's own kernel (the caller counts the last one)
+    VRHI_CUDA(finish_partials(st->s, jobs));
+  }
   return VRHI_OK;
 }
 
@@ -424,8 +513,7 @@ void tape_jit_counters(uint64_t *compiled, uint64_t *launches, int *compiler_ver
 
 // The generated source of a tape, for inspection and for tests that run without a GPU.
 std::string tape_jit_source(const vrhi_tape_params &q) {
-  bool flat = false;
-  return generate(q, &flat);
+  return generate(q, form_of(q), 2);
 }
 
 }  // namespace vrhi

@@ -153,11 +153,32 @@ inline int tape_arity(int op) {
   }
 }
 
+inline bool tape_total(const vrhi_tape_params &q, uint32_t k) { return ((q.total_mask >> k) & 1u) != 0; }
+inline bool tape_mean(const vrhi_tape_params &q, uint32_t k) { return ((q.total_mask >> (8 + k)) & 1u) != 0; }
+
+// Second stage of the reductions whose first stage leaves partial sums (k_rows.cu): job j adds `groups` partial rows of
+// `cols` floats into out[0..cols), scaled.  One launch does up to kMaxFinishJobs of them, as a programmatic dependent
+// of the kernel that wrote the partial rows (the last one launched on the stream).
+constexpr int kMaxFinishJobs = 5;
+struct FinishJobs {
+  struct Job {
+    const float *partial;
+    float *out;
+    double scale;
+    uint64_t cols;
+    uint32_t groups;
+    uint32_t W;           // adjacent columns per block
+    uint32_t last_block;  // one past the job's blocks in the grid
+  } job[kMaxFinishJobs];
+  int n;
+};
+void add_finish_job(FinishJobs *jobs, const float *partial, float *out, uint32_t groups, uint64_t cols, double scale);
+cudaError_t finish_partials(cudaStream_t s, const FinishJobs &jobs);
+
 // Run-time compiled tapes (tape_jit.cpp).  tape_jit_launch returns VRHI_OK (launched), 1 (leave it to
 // the interpreter) or an error code.
 int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *const *in, float *const *out);
 bool tape_jit_available();
-int col_finalize(vrhi_stream_t *st, const float *partial, float *out, uint32_t groups, uint64_t cols, float scale);
 void tape_jit_counters(uint64_t *compiled, uint64_t *launches, int *compiler_version, int *built_version);
 std::string tape_jit_source(const vrhi_tape_params &q);
 
