@@ -281,12 +281,12 @@ struct Planner {
   std::vector<int> stage;
   std::vector<vrhi_buffer> storage;  // node -> buffer holding it (leaves and roots)
   std::map<int, int> op_ids;
-  // Elementwise roots that are summed over the rows inside the map kernel instead of being stored:
-  // root -> the [cols] array that receives the sums.  `folded_nodes`: column-sum nodes that need no
-  // step of their own; `folded_mid`: full sums / means whose first half (the column sum) is done.
-  std::map<int, vrhi_buffer> folded;
+  // Elementwise roots that are summed inside the map kernel instead of being stored: root -> the reduction that
+  // reads it (column sums, full sum or mean) and the array that receives the result.  `folded_nodes`: the
+  // reductions that need no step of their own.
+  struct Fold { int op; vrhi_buffer dst; };
+  std::map<int, Fold> folded;
   std::set<int> folded_nodes;
-  std::map<int, vrhi_buffer> folded_mid;
   int next_order = 0;
 
   bool leaf(int i) const {
@@ -338,6 +338,12 @@ struct Planner {
     a.bytes = g->elems(g->nodes[node].shape) * 4;
     a.arg_class = cls;
     return a;
+  }
+
+  // Output k of the tape is the sum (VRHI_R_SUM_ALL) or mean of its elements.
+  static void mark_total(vrhi_tape_params *P, size_t k, int op) {
+    P->flags |= VRHI_TAPE_FLAG_TOTALS;
+    P->total_mask |= (op == VRHI_R_MEAN_ALL ? 0x101u : 1u) << k;
   }
 
   // Emit one map kernel computing `roots` (same shape, same stage).
@@ -415,16 +421,18 @@ struct Planner {
       auto f = folded.find(roots[k]);
       if (f == folded.end()) {
         s.args.push_back(arg_of(roots[k], VRHI_OUTPUT));
-      } else {  // the map kernel writes the column sums straight into the reduction's array
-        P.colsum_mask |= 1u << k;
+      } else {  // the map kernel writes the sums straight into the reduction's array
+        const bool col = f->second.op == VRHI_R_COL_SUM;
+        if (col) P.colsum_mask |= 1u << k;
+        else mark_total(&P, k, f->second.op);
         vrhi_arg a{};
-        a.buffer = f->second; a.offset = 0; a.bytes = g->cols * 4; a.arg_class = VRHI_OUTPUT;
+        a.buffer = f->second.dst; a.offset = 0; a.bytes = col ? g->cols * 4 : 4; a.arg_class = VRHI_OUTPUT;
         s.args.push_back(a);
       }
     }
     std::ostringstream text;
     bool special = false;
-    if (!(g->flags & 1u) && P.colsum_mask == 0 && shape == VRHI_SHAPE_FULL && roots.size() == 1 && leaf_list.size() == 3 && P.row_vector_mask == 0 && P.col_vector_mask == 0 && P.scalar_mask == 0) {
+    if (!(g->flags & 1u) && (P.colsum_mask | P.total_mask) == 0 && shape == VRHI_SHAPE_FULL && roots.size() == 1 && leaf_list.size() == 3 && P.row_vector_mask == 0 && P.col_vector_mask == 0 && P.scalar_mask == 0) {
       // the map-workload chain, operands of commutative nodes in any order
       special = match_chain(roots[0], leaf_list, &s);
     }
@@ -437,6 +445,7 @@ struct Planner {
            << " instr=" << P.n_instr;
       for (uint32_t k = 0; k < P.n_outputs; ++k)
         if ((P.colsum_mask >> k) & 1u) text << " (output " << k << ": col_sum folded into the kernel)";
+        else if (tape_total(P, k)) text << " (output " << k << (tape_mean(P, k) ? ": mean" : ": sum") << " folded into the kernel)";
     }
     s.text = text.str();
     g->steps.push_back(s);
@@ -649,12 +658,22 @@ struct Planner {
         vrhi_arg flat_in = arg_of(n.a, VRHI_INPUT);
         uint64_t len = g->elems(in_shape);
         vrhi_arg dst = arg_of(i, VRHI_OUTPUT);
-        auto mid_it = folded_mid.find(i);
-        if (mid_it != folded_mid.end()) {  // the map kernel already left the column sums here
-          vrhi_arg mid{}; mid.buffer = mid_it->second; mid.bytes = g->cols * 4; mid.arg_class = VRHI_INPUT;
-          flat_in = mid;
-          len = g->cols;
-        } else if (in_shape == VRHI_SHAPE_FULL) {
+        if (tape_jit_available()) {  // a tape that does nothing but add its input up: one pass, one partial value per block
+          Step s;
+          s.stage = st;
+          s.order = next_order++;
+          VRHI_TRY(vrhi_op_lookup("map_tape", &s.op));
+          vrhi_tape_params P{};
+          P.size = sizeof P; P.n_inputs = 1; P.n_outputs = 1; P.rows = 1; P.cols = len;
+          P.out_value[0] = 0;
+          mark_total(&P, 0, n.op);
+          s.params.assign((unsigned char *)&P, (unsigned char *)&P + sizeof P);
+          s.args = {flat_in, dst};
+          s.text = "map_tape    stage " + std::to_string(st) + " n=" + std::to_string(len) + (n.op == VRHI_R_MEAN_ALL ? " (mean)" : " (flat sum)");
+          g->steps.push_back(s);
+          return VRHI_OK;
+        }
+        if (in_shape == VRHI_SHAPE_FULL) {
           vrhi_buffer t = nullptr;
           VRHI_TRY(vrhi_buffer_create(g->dev, g->cols * 4, VRHI_STORAGE_BUFFER, &t));
           g->temps.push_back(t);
@@ -737,9 +756,9 @@ struct Planner {
           if (!storage[i]) VRHI_TRY(temp_for(i));
         }
       }
-      // A full-size elementwise value whose only reader is a column sum is never written: the map kernel
-      // that computes it adds it up column by column (compiled tapes only).
-      folded.clear(); folded_nodes.clear(); folded_mid.clear();
+      // An elementwise value whose only reader is a column sum, a full sum or a mean is never written: the map
+      // kernel that computes it adds it up (compiled tapes only).
+      folded.clear(); folded_nodes.clear();
       if (tape_jit_available()) {
         // readers that need the value in memory: reductions and softmax (elementwise readers recompute it
         // inside their own kernel from the leaves)
@@ -755,18 +774,10 @@ struct Planner {
           if (!live[i] || n.kind != K_REDUCE) continue;
           if (n.op != VRHI_R_COL_SUM && n.op != VRHI_R_SUM_ALL && n.op != VRHI_R_MEAN_ALL) continue;
           const int a = n.a;
-          if (!is_elementwise(g->nodes[a].kind) || g->nodes[a].shape != VRHI_SHAPE_FULL) continue;
+          if (!is_elementwise(g->nodes[a].kind) || g->nodes[a].shape == VRHI_SHAPE_SCALAR) continue;
           if (readers[a] != 1 || seen_out.count(a) || storage[a] || folded.count(a)) continue;
-          if (n.op == VRHI_R_COL_SUM) {
-            folded[a] = storage[i];
-            folded_nodes.insert(i);
-          } else {  // a full sum is a column sum followed by a flat sum: the first half goes into the kernel
-            vrhi_buffer t = nullptr;
-            VRHI_TRY(vrhi_buffer_create(g->dev, g->cols * 4, VRHI_STORAGE_BUFFER, &t));
-            g->temps.push_back(t);
-            folded[a] = t;
-            folded_mid[i] = t;
-          }
+          folded[a] = Fold{n.op, storage[i]};
+          folded_nodes.insert(i);
         }
       }
       for (int i = 0; i < N; ++i)
