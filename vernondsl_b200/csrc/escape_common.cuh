@@ -13,7 +13,9 @@ namespace vrhi {
 
 struct EscapeDev {
   uint32_t width, height, max_iter;
-  float x0, y0, dx, dy, cr, ci, bound, color_scale;
+  float x0, y0, dx, dy, cr, ci;
+  float limit;               // a pixel has escaped once !(a+b <= limit), whichever test the caller asked for (escape_limit)
+  float color_scale;
   uint32_t chunk_rows, chunk_first, chunk_step;
   uint32_t rows_owned;       // rows this launch computes
   uint32_t tiles_per_row;    // ceil(width / tile), tile = 32 pixels (one per lane) or 64 (two per lane)
@@ -53,11 +55,8 @@ __device__ __forceinline__ void z_advance(float &zr, float &zi, float &a, float 
   }
 }
 
-template <int TEST>
-__device__ __forceinline__ bool escaped(float s, float bound) {
-  if (TEST == VRHI_TEST_NORM2_GT) return !(s <= bound);  // NaN counts as escaped; s > bound otherwise
-  return !(__fsqrt_rn(s) < bound);
-}
+// s = a+b against EscapeDev::limit.  NaN counts as escaped; s > limit otherwise.
+__device__ __forceinline__ bool escaped(float s, float limit) { return !(s <= limit); }
 
 template <int OUT>
 __device__ __forceinline__ void store_count(void *image, size_t pix, uint32_t count, float color_scale) {
@@ -86,6 +85,15 @@ __device__ __forceinline__ void store_wire(uint16_t *wire, uint8_t *bytes, size_
 // Both are no-ops in a launch without the attribute and nothing after it that carries it.
 __device__ __forceinline__ void begin_overlap() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void end_overlap() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Work stealing: the next batch for this warp, n_batches or more when none is left.  A launch makes exactly n_batches
+// fetches that succeed and one that fails per warp, so the wrapping increment leaves the counter at 0 behind the
+// last one and the next launch needs no memset in front of it (a node of its own in a recorded sequence, and the
+// gap before the kernel: measured on B200, a 1080p Mandelbrot frame of 256 steps, 52.8 us with, 50.0 us without).
+// The host keeps n_batches + warps within 32 bits.
+__device__ __forceinline__ uint32_t next_batch(uint32_t *counter, uint32_t n_batches) {
+  return atomicInc(counter, n_batches + gridDim.x * (blockDim.x >> 5) - 1u);
+}
 
 // Launch `kern` on the stream; `overlap`: with the attribute described above.
 template <class Kern, class... Args>
@@ -164,7 +172,8 @@ int launch_pinned(Kern kern, int grid, int per_sm, vrhi_stream_t *st, const Esca
   return VRHI_OK;
 }
 
-// the two-pixels-per-lane kernel (k_escape_pair.cu)
+// the two-pixels-per-lane kernel (k_escape_pair.cu); it takes max_iter from this number of steps on
+constexpr int kPairLeastIter = 64;
 int launch_escape_pair(vrhi_stream_t *st, const vrhi_escape_params &q, const EscapeDev &p, int grid, int per_sm, bool pin, bool overlap,
                        void *image, uint32_t *counter, uint16_t *wire);
 

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256, 4) escape_pair_kernel(EscapeDev p, void *
   const uint32_t FULL = 0xffffffffu;
   float4 *pool = s_pool[warp];
   float2 *poolc = s_c[PER_PIXEL_C ? warp : 0];
-  const float bound = p.bound, x0 = p.x0, dx = p.dx, color_scale = p.color_scale;
+  const float bound = p.limit, x0 = p.x0, dx = p.dx, color_scale = p.color_scale;
   const uint32_t max_iter = p.max_iter, width = p.width;
   const bool transposed = p.transposed != 0;
   const uint32_t fast_limit = max_iter - (uint32_t)U;  // the host guarantees max_iter >= U
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256, 4) escape_pair_kernel(EscapeDev p, void *
   auto intake = [&]() {
     if (tile >= tile_end) {
       uint32_t batch = 0;
-      if (lane == 0) batch = atomicAdd(work_counter, 1u);
+      if (lane == 0) batch = next_batch(work_counter, p.n_batches);
       batch = __shfl_sync(FULL, batch, 0);
       if (batch >= p.n_batches) { fresh = false; return; }
       const uint32_t k = batch / p.batches_per_row;
