@@ -15,6 +15,13 @@ struct EscapeDev {
   uint32_t width, height, max_iter;
   float x0, y0, dx, dy, cr, ci;
   float limit;               // a pixel has escaped once !(a+b <= limit), whichever test the caller asked for (escape_limit)
+  // A pixel goes through blocks of updates without a test only where escape is final: once a+b > limit, every later
+  // a+b is larger still (or Inf/NaN).  |z'| >= |z|^2 - |c|, so with L = limit >= 4 that holds for
+  // |c| <= cmax = min(L - 1.005 sqrt(L), L / 2): each step grows |z| by half a percent at least, and the roundings
+  // of a step by at most 24 units of 2^-24.  In the Mandelbrot iteration z = c after one step, so it also holds for
+  // |c| >= 2.01, escaped or not: |z| >= |c| there and |z'| >= |z| (|z| - 1).  What is left are the constants with
+  // c2_unsafe_lo < |c|^2 < c2_unsafe_hi (none for L >= 4.05, a ring of 0.02 around |c| = 2 for L = 4).
+  float c2_unsafe_lo, c2_unsafe_hi;
   float color_scale;
   uint32_t chunk_rows, chunk_first, chunk_step;
   uint32_t rows_owned;       // rows this launch computes
@@ -26,6 +33,11 @@ struct EscapeDev {
   float neg_zero;            // -0.0f, set by the host: an addend the assembler cannot fold (k_escape_pair.cu)
   uint8_t *bytes;            // optional third copy of every count, min(count, 255), at the same pixel index (nullptr: none)
 };
+
+__device__ __forceinline__ bool unsafe_constant(const EscapeDev &p, float cr, float ci) {
+  const float c2 = __fmaf_rn(cr, cr, __fmul_rn(ci, ci));
+  return c2 > p.c2_unsafe_lo && c2 < p.c2_unsafe_hi;
+}
 
 // Step primitives.  EXACT keeps a = zr*zr and b = zi*zi alongside z so that one update costs six
 // instructions; FAST lets multiply-adds fuse (four instructions per update) and is a different,
@@ -58,6 +70,70 @@ __device__ __forceinline__ void z_advance(float &zr, float &zi, float &a, float 
 // s = a+b against EscapeDev::limit.  NaN counts as escaped; s > limit otherwise.
 __device__ __forceinline__ bool escaped(float s, float limit) { return !(s <= limit); }
 
+// TWO PIXELS IN ONE REGISTER PAIR.  A packed operation rounds each half exactly like the scalar operation, so the counts
+// are the same bits as the one-pixel-per-lane kernel and the CPU statement.  One trap: the
+// assembler contracts mul.rn.f32x2 followed by add/sub.rn.f32x2 into a fused multiply-add (it does
+// so even through fma(x, y, -0.0) with a literal -0.0), which changes the rounding of
+// (zr*zr - zi*zi).  Every product here is therefore fma(x, y, nz) with nz = -0.0 read from the
+// kernel parameters, a value the assembler cannot see: x*y + (-0.0) is x*y rounded once, sign of
+// zero included, and an fma feeding an add is never contracted further.
+typedef unsigned long long f32x2;  // two binary32 values in one 64-bit register; "lo" is slot 0
+
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
+// lo half from `n` where c0 holds, else from `o`; hi half likewise with c1
+__device__ __forceinline__ f32x2 select2(bool c0, bool c1, f32x2 n, f32x2 o) {
+  float nl, nh, ol, oh;
+  unpack2(n, nl, nh);
+  unpack2(o, ol, oh);
+  return pack2(c0 ? nl : ol, c1 ? nh : oh);
+}
+
+// The step primitives of escape_common.cuh on pairs; `nz` is the invisible -0.0 (see the top).
+template <int MODE>
+__device__ __forceinline__ void pair_squares(f32x2 zr, f32x2 zi, f32x2 nz, f32x2 &a, f32x2 &b) {
+  if (MODE == VRHI_ESCAPE_EXACT) { a = fma2(zr, zr, nz); b = fma2(zi, zi, nz); }
+}
+template <int MODE>
+__device__ __forceinline__ f32x2 pair_norm2(f32x2 zr, f32x2 zi, f32x2 a, f32x2 b, f32x2 nz) {
+  if (MODE == VRHI_ESCAPE_EXACT) return add2(a, b);
+  return fma2(zi, zi, fma2(zr, zr, nz));
+}
+template <int MODE>
+__device__ __forceinline__ void pair_advance(f32x2 &zr, f32x2 &zi, f32x2 &a, f32x2 &b, f32x2 cr, f32x2 ci, f32x2 nz, f32x2 two) {
+  if (MODE == VRHI_ESCAPE_EXACT) {
+    const f32x2 t = fma2(zr, zi, nz);
+    zi = fma2(two, t, ci);
+    zr = add2(sub2(a, b), cr);
+    a = fma2(zr, zr, nz);
+    b = fma2(zi, zi, nz);
+  } else {
+    const f32x2 nzi = fma2(add2(zr, zr), zi, ci);
+    zr = fma2(zr, zr, fma2(neg2(zi), zi, cr));
+    zi = nzi;
+  }
+}
+
 template <int OUT>
 __device__ __forceinline__ void store_count(void *image, size_t pix, uint32_t count, float color_scale) {
   if (OUT == VRHI_OUT_COUNT_U32)
@@ -75,6 +151,18 @@ __device__ __forceinline__ void store_count(void *image, size_t pix, uint32_t co
 __device__ __forceinline__ void store_wire(uint16_t *wire, uint8_t *bytes, size_t pix, uint32_t count) {
   wire[pix] = (uint16_t)count;
   if (bytes) bytes[pix] = (uint8_t)min(count, 255u);
+}
+
+// From `count` steps done: the step-by-step loop to the end.
+template <int MODE>
+__device__ __forceinline__ uint32_t escape_count(float zr, float zi, float cr, float ci, float limit, uint32_t count, uint32_t max_iter) {
+  float a = 0.f, b = 0.f;
+  z_squares<MODE>(zr, zi, a, b);
+  while (!escaped(z_norm2<MODE>(zr, zi, a, b), limit) && count < max_iter) {
+    z_advance<MODE>(zr, zi, a, b, cr, ci);
+    ++count;
+  }
+  return count;
 }
 
 // A launch that its caller declared independent of the launches before it is started with the
@@ -172,9 +260,11 @@ int launch_pinned(Kern kern, int grid, int per_sm, vrhi_stream_t *st, const Esca
   return VRHI_OK;
 }
 
-// the two-pixels-per-lane kernel (k_escape_pair.cu); it takes max_iter from this number of steps on
-constexpr int kPairLeastIter = 64;
+// the regrouping kernel (k_escape_pair.cu); it needs max_iter >= 12, the length of its blocks and of its intake
 int launch_escape_pair(vrhi_stream_t *st, const vrhi_escape_params &q, const EscapeDev &p, int grid, int per_sm, bool pin, bool overlap,
                        void *image, uint32_t *counter, uint16_t *wire);
+
+// the kernel for launches with little to regroup (k_escape_block.cu)
+int launch_escape_block(vrhi_stream_t *st, const vrhi_escape_params &q, EscapeDev p, bool overlap, void *image, uint16_t *wire);
 
 }  // namespace vrhi

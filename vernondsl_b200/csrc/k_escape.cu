@@ -58,14 +58,7 @@ __global__ void __launch_bounds__(256) escape_checked_kernel(EscapeDev p, void *
       } else {
         zr = p.transposed ? y : x; zi = p.transposed ? x : y; cr = p.cr; ci = p.ci;
       }
-      uint32_t count = 0;
-      float a = 0.f, b = 0.f;
-      z_squares<MODE>(zr, zi, a, b);
-      for (;;) {
-        if (escaped(z_norm2<MODE>(zr, zi, a, b), p.limit) || count >= p.max_iter) break;
-        z_advance<MODE>(zr, zi, a, b, cr, ci);
-        ++count;
-      }
+      const uint32_t count = escape_count<MODE>(zr, zi, cr, ci, p.limit, 0u, p.max_iter);
       store_count<OUT>(image, row_base + i, count, p.color_scale);
       if (wire) store_wire(wire, p.bytes, row_base + i, count);
     }
@@ -157,12 +150,52 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
   static const int env_batch = [] { const char *e = getenv("VRHI_ESCAPE_BATCH"); return e ? atoi(e) : 0; }();
   static const int env_per_sm = [] { const char *e = getenv("VRHI_ESCAPE_CTAS_PER_SM"); return e ? atoi(e) : 0; }();
   const int sms = st->dev->prop.multiProcessorCount;
-  // The regrouping kernels take what their exactness argument covers; everything else, and callers
-  // that ask for it, runs the step-by-step kernel.
+  // The kernels with unchecked blocks take what their exactness argument covers (EscapeDev::c2_unsafe_lo); everything
+  // else, and callers that ask for it, runs the step-by-step kernel.
+  const double root = sqrt((double)p.limit), cmax = fmin(p.limit - 1.005 * root, 0.5 * p.limit);
   const double c2 = (double)q.cr * q.cr + (double)q.ci * q.ci;
-  const bool regroup_ok = p.limit >= 4.0f && p.limit < 3.0e38f &&
-                          q.max_iter >= (uint32_t)kPairLeastIter && q.max_iter <= (1u << 30) && (uint64_t)q.width * q.height <= 0xffffffffull &&
-                          (q.kind == VRHI_ESCAPE_MANDELBROT || c2 <= 2.25) && !(q.flags & VRHI_ESCAPE_FLAG_CHECKED_ONLY);
+  p.c2_unsafe_lo = (float)(cmax * cmax * (1.0 - 1e-6));
+  p.c2_unsafe_hi = 4.05f;
+  const bool blocks_ok = p.limit >= 4.0f && p.limit < 3.0e38f && q.max_iter <= (1u << 30) &&
+                         (q.kind == VRHI_ESCAPE_MANDELBROT || sqrt(c2) <= cmax) && !(q.flags & VRHI_ESCAPE_FLAG_CHECKED_ONLY);
+  // Two kernels with unchecked blocks.  The regrouping one (k_escape_pair.cu) pays about 2 us per tile and warp for intake
+  // and pool and then loses nothing to pixels that outlive their neighbours; the block kernel (k_escape_block.cu) runs a
+  // warp as long as its slowest pixel.  So regroup where pixels may run long and every warp sees many tiles.  Measured on B200,
+  // regrouping against blocks, Julia / Mandelbrot in us:
+  //   640 x 320     256 steps: 13.3 vs 10.9 / 13.4 vs 9.5       1024: 30.4 vs 31.3 / 42.8 vs 30.4
+  //   1920 x 1080   128: 31.1 vs 27.4 / 34.6 vs 30.4            256: 36.5 vs 43.3 / 48.9 vs 47.4     1024: 55 vs 103 / 143 vs 151
+  //   4096 x 4096   64: 107 vs 106 / 141 vs 127                 128: 130 vs 154 / 183 vs 188         256: 164 vs 251 / 283 vs 303
+  const uint64_t pixels = (uint64_t)q.width * p.rows_owned;
+  //   128 x 64      256: 7.2 vs 6.8 / 7.4 vs 7.0                1024: 14.9 vs 19.4 / 18.3 vs 23.6 (one tile per warp: the
+  //                 length of a warp's chain of blocks and votes is all there is)
+  const uint32_t regroup_from = pixels >= (4ull << 20) ? 96u : pixels >= (512ull << 10) ? 192u : pixels >= (64ull << 10) ? 0xffffffffu : 512u;
+  bool regroup_ok = blocks_ok && q.max_iter >= regroup_from && (uint64_t)q.width * q.height <= 0xffffffffull;
+  // The regrouping kernel's work counter lives in the stream's scratch.  A launch of 64 steps or more with the a+b test asks
+  // for it whichever kernel is chosen, so that recording one on a stream that has never run one is refused whatever the
+  // image's size; any other launch is recorded there with the kernel that needs none.
+  const bool asks = blocks_ok && q.test == VRHI_TEST_NORM2_GT && q.max_iter >= 64u && (q.kind == VRHI_ESCAPE_MANDELBROT || c2 <= 2.25);
+  if (asks) VRHI_TRY(stream_arena(st, 0, nullptr, nullptr));
+  if (regroup_ok && !st->arena) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    VRHI_CUDA(cudaStreamIsCapturing(st->s, &cap));
+    regroup_ok = cap == cudaStreamCaptureStatusNone;
+  }
+  // A launch declared independent of the k launches before it (flags, bits 8-10) may begin before they end.
+  // Such launches form runs: the first of a run is ordered behind everything earlier on the stream, each
+  // further one is started with the overlap attribute, and a run ends where a launch is no longer independent
+  // of the run's first (run length > k) or anything else happens on the stream.  Launch i of a run therefore
+  // only ever runs beside launches it was declared independent of.  The launches of a run take their work from
+  // counters of their own; every launch leaves its counter at 0 (next_batch).
+  const uint32_t independent_of = (q.flags & VRHI_ESCAPE_FLAG_INDEPENDENT_MASK) >> VRHI_ESCAPE_FLAG_INDEPENDENT_SHIFT;
+  const int run = st->escape_chain;  // launches of the current run so far
+  const bool overlap = independent_of != 0 && run >= 1 && (uint32_t)run <= independent_of && run < 8;
+  const int run_after = independent_of == 0 ? 0 : overlap ? run + 1 : 1;
+  if (blocks_ok && !regroup_ok && p.rows_owned <= 1u << 31) {
+    VRHI_TRY(launch_escape_block(st, q, p, overlap, args[0].ptr, wire));
+    VRHI_TRY(post_launch(st, "escape_time (blocks)"));
+    st->escape_chain = run_after;
+    return VRHI_OK;
+  }
   const bool pair = regroup_ok;               // two pixels per lane (k_escape_pair.cu)
   const uint32_t tile_px = pair ? 64u : 32u;  // pixels a warp takes in per intake trip
   p.tiles_per_row = (q.width + tile_px - 1) / tile_px;
@@ -186,25 +219,14 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
 
   uint64_t warps_needed = nb;
   int grid = (int)((warps_needed + 7) / 8 < (uint64_t)sms * 8 ? (warps_needed + 7) / 8 : (uint64_t)sms * 8);
-  // A frame of a few batches per warp (the 640 x 320 frame of fractal.py:7-8 is one) is dealt out
-  // statically: resetting a work counter would be a second node per frame and cost as much as the frame.
+  // a small image's batches are dealt out: fetching them from the counter would be most of the work
   const bool dealt = !regroup_ok && nb <= (uint64_t)grid * 8 * 4;
-  // A launch declared independent of the k launches before it (flags, bits 8-10) may begin before they end.
-  // Such launches form runs: the first of a run is ordered behind everything earlier on the stream, each
-  // further one is started with the overlap attribute, and a run ends where a launch is no longer independent
-  // of the run's first (run length > k) or anything else happens on the stream.  Launch i of a run therefore
-  // only ever runs beside launches it was declared independent of.  The launches of a run take their work from
-  // counters of their own; every launch leaves its counter at 0 (next_batch).
-  const uint32_t independent_of = (q.flags & VRHI_ESCAPE_FLAG_INDEPENDENT_MASK) >> VRHI_ESCAPE_FLAG_INDEPENDENT_SHIFT;
-  const int run = st->escape_chain;  // launches of the current run so far
-  const bool overlap = independent_of != 0 && run >= 1 && (uint32_t)run <= independent_of && run < 8;
   uint32_t *counter = nullptr;
   if (!dealt) {
     uint32_t *ctrl = nullptr;
     VRHI_TRY(stream_arena(st, 0, &ctrl, nullptr));
     counter = independent_of == 0 ? ctrl + CTRL_WORK0 : ctrl + CTRL_ESCAPE_RING + (overlap ? run : 0);
   }
-  const int run_after = independent_of == 0 ? 0 : overlap ? run + 1 : 1;
   // a grid whose failing fetches would carry the counter past 32 bits (see next_batch) is made smaller
   const uint64_t most_grid = (0xffffffffull - nb) / 8;
   if ((uint64_t)grid > most_grid) grid = (int)most_grid;
@@ -214,13 +236,14 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
     // each warp then owns enough tiles to keep its pool busy and the drain at the end is shorter.
     uint64_t ctas = (nb + 7) / 8;
     const uint64_t px_total = (uint64_t)p.tiles_per_row * tile_px * p.rows_owned;
-    // Launches of less than a quarter of the 16384^2 image are usually one of several per step (a rank's rows
+    // Launches of less than 16 Mi pixels are usually one of several per step (a rank's rows
     // computed group by group, frames of a sequence): with 2 blocks per SM and no pinning the blocks of the next
     // launch move in beside the draining ones (measured, four launches of 1/32 of that image each on two streams:
     // 0.39 ms against 0.45 ms with 4 pinned blocks per SM).
     // Larger launches: 3 blocks per SM, pinned (measured on the 16384^2 image with 1024-pixel batches: 2.133 ms
-    // against 2.145 ms with 4; with 512-pixel batches 3, 4 and 5 gave 2.170, 2.164 and 2.165 ms).
-    uint64_t per_sm = px_total < (64ull << 20) ? 2 : 3;
+    // against 2.145 ms with 4; with 512-pixel batches 3, 4 and 5 gave 2.170, 2.164 and 2.165 ms; 4096 x 4096, 128 steps:
+    // Julia 129.6 us with 3, 136.5 with 2, Mandelbrot 182.8 and 190.9).
+    uint64_t per_sm = px_total < (16ull << 20) ? 2 : 3;
     if (env_per_sm >= 1 && env_per_sm <= 6) per_sm = (uint64_t)env_per_sm;
     const uint64_t cap = (uint64_t)sms * per_sm;
     grid = (int)(ctas < cap ? ctas : cap);

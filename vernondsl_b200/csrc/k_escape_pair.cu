@@ -34,13 +34,7 @@
 // other resident warps runs in the slots between.  Measured on B200, 16384^2 Julia image: 2.49 ms
 // with one pixel per lane, 2.17 ms with two; 699 M -> 465 M issued instructions on the 8192^2 image.
 //
-// Exactness.  A packed operation rounds each half exactly like the scalar operation, so the counts
-// are the same bits as the one-pixel-per-lane kernel and the CPU statement.  One trap: the
-// assembler contracts mul.rn.f32x2 followed by add/sub.rn.f32x2 into a fused multiply-add (it does
-// so even through fma(x, y, -0.0) with a literal -0.0), which changes the rounding of
-// (zr*zr - zi*zi).  Every product here is therefore fma(x, y, nz) with nz = -0.0 read from the
-// kernel parameters, a value the assembler cannot see: x*y + (-0.0) is x*y rounded once, sign of
-// zero included, and an fma feeding an add is never contracted further.
+// Exactness of the packed operations: see escape_common.cuh.
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -49,63 +43,6 @@
 #include "escape_common.cuh"
 
 namespace vrhi {
-
-typedef unsigned long long f32x2;  // two binary32 values in one 64-bit register; "lo" is slot 0
-
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
-// lo half from `n` where c0 holds, else from `o`; hi half likewise with c1
-__device__ __forceinline__ f32x2 select2(bool c0, bool c1, f32x2 n, f32x2 o) {
-  float nl, nh, ol, oh;
-  unpack2(n, nl, nh);
-  unpack2(o, ol, oh);
-  return pack2(c0 ? nl : ol, c1 ? nh : oh);
-}
-
-// The step primitives of escape_common.cuh on pairs; `nz` is the invisible -0.0 (see the top).
-template <int MODE>
-__device__ __forceinline__ void pair_squares(f32x2 zr, f32x2 zi, f32x2 nz, f32x2 &a, f32x2 &b) {
-  if (MODE == VRHI_ESCAPE_EXACT) { a = fma2(zr, zr, nz); b = fma2(zi, zi, nz); }
-}
-template <int MODE>
-__device__ __forceinline__ f32x2 pair_norm2(f32x2 zr, f32x2 zi, f32x2 a, f32x2 b, f32x2 nz) {
-  if (MODE == VRHI_ESCAPE_EXACT) return add2(a, b);
-  return fma2(zi, zi, fma2(zr, zr, nz));
-}
-template <int MODE>
-__device__ __forceinline__ void pair_advance(f32x2 &zr, f32x2 &zi, f32x2 &a, f32x2 &b, f32x2 cr, f32x2 ci, f32x2 nz, f32x2 two) {
-  if (MODE == VRHI_ESCAPE_EXACT) {
-    const f32x2 t = fma2(zr, zi, nz);
-    zi = fma2(two, t, ci);
-    zr = add2(sub2(a, b), cr);
-    a = fma2(zr, zr, nz);
-    b = fma2(zi, zi, nz);
-  } else {
-    const f32x2 nzi = fma2(add2(zr, zr), zi, ci);
-    zr = fma2(zr, zr, fma2(neg2(zi), zi, cr));
-    zi = nzi;
-  }
-}
 
 constexpr int kPairPool = 128;  // pool entries per warp: a refill wants up to 64, an intake trip adds up to 64
 
@@ -186,26 +123,19 @@ __global__ void __launch_bounds__(256, 4) escape_pair_kernel(EscapeDev p, void *
       fc0 += l0 ? 1u : 0u;
       fc1 += l1 ? 1u : 0u;
     }
-    if (PER_PIXEL_C) {
-      // pixels whose own constant is too large for unchecked blocks are finished here, step by step
-      float c0r, c1r, c0i, c1i;
+    if (PER_PIXEL_C && p.c2_unsafe_lo < p.c2_unsafe_hi) {
+      // pixels whose own constant rules out unchecked blocks are finished here, step by step (on the real axis they run
+      // to max_iter: about 30 cycles a step, where a packed step with a vote took 250)
+      float c0r, c1r, c0i, c1i, z0r, z1r, z0i, z1i;
       unpack2(FCR, c0r, c1r);
       unpack2(FCI, c0i, c1i);
-      bool slow0 = l0 && !(__fmaf_rn(c0r, c0r, __fmul_rn(c0i, c0i)) <= 2.25f);
-      bool slow1 = l1 && !(__fmaf_rn(c1r, c1r, __fmul_rn(c1i, c1i)) <= 2.25f);
-      while (__any_sync(FULL, slow0 || slow1)) {
-        float s0, s1;
-        unpack2(pair_norm2<MODE>(FZR, FZI, FA, FB, NZ), s0, s1);
-        if (slow0 && (!(s0 <= bound) || fc0 >= max_iter)) { slow0 = false; l0 = false; }
-        if (slow1 && (!(s1 <= bound) || fc1 >= max_iter)) { slow1 = false; l1 = false; }
-        f32x2 NR = FZR, NI = FZI, NA = FA, NB = FB;
-        pair_advance<MODE>(NR, NI, NA, NB, FCR, FCI, NZ, TWO);
-        // only the slots being finished here move; survivors on their way to the pool keep their state
-        FZR = select2(slow0, slow1, NR, FZR);
-        FZI = select2(slow0, slow1, NI, FZI);
-        if (MODE == VRHI_ESCAPE_EXACT) { FA = select2(slow0, slow1, NA, FA); FB = select2(slow0, slow1, NB, FB); }
-        fc0 += slow0 ? 1u : 0u;
-        fc1 += slow1 ? 1u : 0u;
+      const bool slow0 = l0 && unsafe_constant(p, c0r, c0i), slow1 = l1 && unsafe_constant(p, c1r, c1i);
+      if (__any_sync(FULL, slow0 || slow1)) {
+        unpack2(FZR, z0r, z1r);
+        unpack2(FZI, z0i, z1i);
+        if (slow0) { fc0 = escape_count<MODE>(z0r, z0i, c0r, c0i, bound, fc0, max_iter); l0 = false; }
+        if (slow1) { fc1 = escape_count<MODE>(z1r, z1i, c1r, c1i, bound, fc1, max_iter); l1 = false; }
+        __syncwarp();
       }
     }
     if (valid0 && !l0) finish(row_base + i0, fc0);
