@@ -4,9 +4,8 @@ to run with its import line changed (``import vernondsl_b200.lang as ti``) and i
 Surface (reference lines): ``init`` (fractal.py:5), ``field`` (:8), ``@func`` (:11), ``Vector`` (:13),
 ``@kernel`` (:16), the struct-for ``for i, j in field`` (:18), ``cos`` (:19), ``.norm()`` (:22).
 
-A kernel is not interpreted element by element anywhere.  Its Python source is parsed once and, at
-each call, walked with symbolic values to recognise one of two shapes; the result is ONE launch of
-a hand-written CUDA kernel:
+A kernel is not interpreted element by element anywhere.  Its Python source is parsed once and walked with
+symbolic values to recognise one of two shapes; the result is ONE launch of a hand-written CUDA kernel:
 
 * the escape-time shape of fractal.py:18-25 -- pixel-dependent start or constant, a
   ``while z.norm() < R and it < N`` (or ``z.norm_sqr() <= R``) loop whose body is the quadratic map
@@ -16,6 +15,11 @@ a hand-written CUDA kernel:
   launch (one fused kernel).
 
 Anything else raises ``LangError``: there is no interpreter fallback.
+
+The walk takes a few hundred microseconds, many times what a frame takes on the device.  Where a kernel's arguments
+only enter the constant of the escape-time shape (the phase of fractal.py:19), what the walk found is kept with
+everything it read from outside the kernel -- names of the enclosing scopes and of modules, shapes of fields -- and
+a later call that finds all of that unchanged only evaluates the constant (``_Plan``).
 
 Index arithmetic: an expression affine in the loop indices, such as ``(i / n - 1) * 2``, is
 evaluated exactly (rational arithmetic) to ``origin + index * step``, and origin and step are then
@@ -27,9 +31,12 @@ fractal.py:13.
 from __future__ import annotations
 
 import ast
+import builtins
 import inspect
 import math
+import operator
 import textwrap
+import types
 from fractions import Fraction
 from typing import Any, Dict, List, Optional, Tuple
 
@@ -145,6 +152,8 @@ class Sym:
 
     # operator overloads build the tree
     def _b(self, op, o, swap=False):
+        if isinstance(o, _Uniform):
+            raise _Depends()
         o = o if isinstance(o, Sym) else Sym("const", value=o)
         return Sym(op, (o, self) if swap else (self, o))
 
@@ -163,6 +172,50 @@ class Sym:
         if k == 2:
             return Sym("mul", (self, self))
         raise LangError("only ** 2 is supported")
+
+
+class _Depends(Exception):
+    """A kernel argument reaches something other than the constant of the escape-time shape."""
+
+
+class _Uniform:
+    """A scalar computed from the kernel's arguments: its value in this call, and how to compute it in another.
+    Anything but scalar arithmetic with it raises ``_Depends``."""
+    __slots__ = ("value", "of")
+    __array_ufunc__ = None      # a numpy scalar on the left hands the operation to __radd__ and its like
+
+    def __init__(self, value, of):
+        self.value, self.of = value, of
+
+    @staticmethod
+    def apply(f, *xs):
+        if not all(isinstance(x, _Uniform) or _is_num(x) for x in xs):
+            raise _Depends()
+        fs = [x.of if isinstance(x, _Uniform) else (lambda args, x=x: x) for x in xs]
+        value = f(*[x.value if isinstance(x, _Uniform) else x for x in xs])
+        if len(fs) == 1:
+            g, = fs
+            return _Uniform(value, lambda args: f(g(args)))
+        g, h = fs
+        return _Uniform(value, lambda args: f(g(args), h(args)))
+
+    def __add__(self, o): return self.apply(operator.add, self, o)
+    def __radd__(self, o): return self.apply(operator.add, o, self)
+    def __sub__(self, o): return self.apply(operator.sub, self, o)
+    def __rsub__(self, o): return self.apply(operator.sub, o, self)
+    def __mul__(self, o): return self.apply(operator.mul, self, o)
+    def __rmul__(self, o): return self.apply(operator.mul, o, self)
+    def __truediv__(self, o): return self.apply(operator.truediv, self, o)
+    def __rtruediv__(self, o): return self.apply(operator.truediv, o, self)
+    def __pow__(self, o): return self.apply(operator.pow, self, o)
+    def __rpow__(self, o): return self.apply(operator.pow, o, self)
+    def __neg__(self): return self.apply(operator.neg, self)
+
+    def _depends(self, *_):
+        raise _Depends()
+
+    __float__ = __int__ = __index__ = __bool__ = __abs__ = __hash__ = _depends
+    __eq__ = __ne__ = __lt__ = __le__ = __gt__ = __ge__ = __getattr__ = _depends
 
 
 def _is_num(v) -> bool:
@@ -198,6 +251,8 @@ def _unary(name, pyfn):
     def f(x):
         if isinstance(x, Sym):
             return Sym(name, (x,))
+        if isinstance(x, _Uniform):
+            return _Uniform.apply(f, x)
         return f32(pyfn(f32(x)))  # uniform scalar: binary32 on the host
     return f
 
@@ -316,34 +371,111 @@ def _poly(e, names) -> Optional[Dict[Tuple[int, int], Fraction]]:
 # ------------------------------------------------------------------------------------------------
 # The walker: a small evaluator over the subset of Python that kernel bodies use.
 
+def _parse(fn) -> ast.FunctionDef:
+    tree = ast.parse(textwrap.dedent(inspect.getsource(fn)))
+    return next(n for n in tree.body if isinstance(n, ast.FunctionDef))
+
+
+class _Reads:
+    """What a walk read from outside the kernel, for a later call to compare."""
+    _ABSENT = object()
+
+    def __init__(self):
+        self.cells: List[Tuple[Any, Any]] = []              # (closure cell, content)
+        self.names: List[Tuple[dict, str, Any]] = []        # (namespace, name, value or _ABSENT)
+        self.fields: Dict[int, Tuple[Any, tuple, Any]] = {}  # id -> (field, shape, dtype); holding the field keeps its id
+
+    def value(self, v):
+        """Only values that say all there is to know by being the same object, or an equal number."""
+        if isinstance(v, Field):
+            self.fields[id(v)] = (v, v.shape, v.dtype)
+        elif not (_is_num(v) or isinstance(v, (_Func, types.ModuleType)) or any(v is f for f in _known())):
+            raise _Depends()
+        return v
+
+    def cell(self, cell):
+        v = cell.cell_contents
+        self.cells.append((cell, self.value(v)))
+        return v
+
+    def name(self, namespace, name):
+        if name not in namespace:
+            self.names.append((namespace, name, self._ABSENT))
+            return self._ABSENT
+        v = namespace[name]
+        self.names.append((namespace, name, self.value(v)))
+        return v
+
+    @staticmethod
+    def _same(v, w) -> bool:
+        # equal numbers of one type are the same number, but for 0.0 and -0.0; a NaN is only the same as itself
+        return v is w or (type(v) is type(w) and _is_num(v) and v == w and v != 0)
+
+    def unchanged(self) -> bool:
+        try:
+            for cell, v in self.cells:
+                c = cell.cell_contents
+                if c is not v and not self._same(c, v):
+                    return False
+        except ValueError:      # the cell was emptied
+            return False
+        for namespace, name, v in self.names:
+            c = namespace.get(name, self._ABSENT)
+            if c is not v and not self._same(c, v):
+                return False
+        for f, shape, dtype in self.fields.values():
+            if f.shape != shape or f.dtype != dtype:
+                return False
+        return True
+
+
+def _known():
+    """The functions of this module a kernel may call."""
+    return (Vector, cos, sin, sqrt, exp, log, tanh)
+
+
 class _Walker:
-    def __init__(self, fn, call_args):
-        self.fn = fn
-        src = textwrap.dedent(inspect.getsource(fn))
-        tree = ast.parse(src)
-        self.fdef = next(n for n in tree.body if isinstance(n, ast.FunctionDef))
+    """``reads``: where what the walk reads from outside is written down, or None; the arguments are then ``_Uniform``."""
+
+    def __init__(self, fn, fdef, call_args, reads: Optional[_Reads] = None):
+        self.fn, self.fdef, self.reads = fn, fdef, reads
         self.globals = fn.__globals__
-        closure = {}
-        if fn.__closure__:
-            closure = {name: cell.cell_contents for name, cell in zip(fn.__code__.co_freevars, fn.__closure__)}
-        self.env: Dict[str, Any] = dict(closure)
-        params = [a.arg for a in self.fdef.args.args]
-        if len(params) != len(call_args):
-            raise TypeError(f"{fn.__name__}() takes {len(params)} arguments, {len(call_args)} given")
-        for name, value, a in zip(params, call_args, self.fdef.args.args):
-            ann = a.annotation
-            is_float = isinstance(ann, ast.Name) and ann.id == "float"
-            self.env[name] = f32(value) if is_float or isinstance(value, float) else value
+        self.closure = dict(zip(fn.__code__.co_freevars, fn.__closure__)) if fn.__closure__ else {}
+        # every enclosing name is part of the environment, as a kernel body may not rebind one it has not bound before
+        self.env: Dict[str, Any] = {} if reads else {name: cell.cell_contents for name, cell in self.closure.items()}
+        values = _bind(fn, fdef, call_args)
+        for k, (a, value) in enumerate(zip(fdef.args.args, values)):
+            if reads:
+                if not _is_num(value):
+                    raise _Depends()
+                value = _Uniform(value, operator.itemgetter(k))
+            self.env[a.arg] = value
 
     def lookup(self, name):
         if name in self.env:
             return self.env[name]
-        if name in self.globals:
+        if self.reads:
+            if name in self.closure:
+                return self.reads.cell(self.closure[name])
+            for namespace in (self.globals, vars(builtins)):
+                v = self.reads.name(namespace, name)
+                if v is not _Reads._ABSENT:
+                    return v
+        elif name in self.globals:
             return self.globals[name]
-        import builtins
-        if hasattr(builtins, name):
+        elif hasattr(builtins, name):
             return getattr(builtins, name)
         raise LangError(f"name {name!r} is not defined in the kernel's scope")
+
+    def attribute(self, base, attr):
+        if self.reads:
+            if not isinstance(base, types.ModuleType):
+                raise _Depends()
+            v = self.reads.name(vars(base), attr)
+            if v is not _Reads._ABSENT:
+                return v
+            raise _Depends()
+        return getattr(base, attr)
 
     def ev(self, node):
         if isinstance(node, ast.Constant):
@@ -351,7 +483,7 @@ class _Walker:
         if isinstance(node, ast.Name):
             return self.lookup(node.id)
         if isinstance(node, ast.Attribute):
-            return getattr(self.ev(node.value), node.attr)
+            return self.attribute(self.ev(node.value), node.attr)
         if isinstance(node, ast.List) or isinstance(node, ast.Tuple):
             return [self.ev(e) for e in node.elts]
         if isinstance(node, ast.UnaryOp):
@@ -377,12 +509,16 @@ class _Walker:
             idx = self.ev(node.slice)
             if isinstance(base, Field):
                 return self.field_read(base, idx if isinstance(idx, list) else [idx])
+            if self.reads and not isinstance(base, Vector):
+                raise _Depends()
             return base[idx]
         if isinstance(node, ast.Call):
             f = self.ev(node.func)
             args = [self.ev(a) for a in node.args]
             if isinstance(f, _Func):
-                return f.inline(args)
+                return f.inline(args, self.reads)
+            if self.reads and not any(f is g for g in _known()):
+                raise _Depends()
             return f(*args)
         raise LangError(f"unsupported expression: {ast.dump(node)[:80]}")
 
@@ -402,12 +538,11 @@ class _Func:
 
     def __init__(self, fn):
         self.fn = fn
-        src = textwrap.dedent(inspect.getsource(fn))
-        self.fdef = next(n for n in ast.parse(src).body if isinstance(n, ast.FunctionDef))
+        self.fdef = _parse(fn)
 
-    def inline(self, args):
+    def inline(self, args, reads: Optional[_Reads] = None):
         w = _Walker.__new__(_Walker)
-        w.fn, w.fdef, w.globals = self.fn, self.fdef, self.fn.__globals__
+        w.fn, w.fdef, w.globals, w.closure, w.reads = self.fn, self.fdef, self.fn.__globals__, {}, reads
         w.env = {a.arg: v for a, v in zip(self.fdef.args.args, args)}
         for stmt in self.fdef.body:
             if isinstance(stmt, ast.Return):
@@ -428,9 +563,41 @@ def func(fn):
     return _Func(fn)
 
 
+def _bind(fn, fdef, call_args) -> list:
+    """The kernel's arguments as its body sees them: floats in binary32."""
+    params = fdef.args.args
+    if len(params) != len(call_args):
+        raise TypeError(f"{fn.__name__}() takes {len(params)} arguments, {len(call_args)} given")
+    return [f32(v) if (isinstance(a.annotation, ast.Name) and a.annotation.id == "float") or isinstance(v, float) else v
+            for a, v in zip(params, call_args)]
+
+
+class _Plan:
+    """An escape-time launch as a walk with ``_Uniform`` arguments found it: the parameter block, how the constant's two
+    components follow from the arguments, and what the walk read from outside the kernel."""
+
+    def __init__(self, reads: _Reads, field: Field, params, constant, text: str):
+        self.reads, self.field, self.params, self.constant, self.text = reads, field, params, constant, text
+
+    def instance(self, fn, fdef, call_args):
+        """The parameter block for other arguments, or None where the walk has to be repeated."""
+        if not self.reads.unchanged():
+            return None
+        values = _bind(fn, fdef, call_args)
+        if not all(type(v) in (f32, int, float) for v in values):
+            return None
+        c = [x if of is None else float(f32(float(of(values)))) for x, of in zip((self.params.cr, self.params.ci), self.constant)]
+        if not (math.isfinite(c[0]) and math.isfinite(c[1])):
+            return None
+        p = type(self.params).from_buffer_copy(self.params)
+        p.cr, p.ci = c
+        p.flags = (p.flags & ~0x700) | (_state["independent_of"] << 8)
+        return p
+
+
 class Kernel:
-    """@ti.kernel (fractal.py:16).  Calling it plans and launches; nothing is cached across calls
-    except the parsed source, so changing a uniform per frame (fractal.py:30-31) just relaunches."""
+    """@ti.kernel (fractal.py:16).  Calling it plans and launches; changing a uniform per frame (fractal.py:30-31)
+    relaunches, with the plan of the call before where nothing the plan rests on has changed."""
 
     def __init__(self, fn):
         self.fn = fn
@@ -438,10 +605,32 @@ class Kernel:
         self.last_plan: Optional[str] = None
         self.last_params = None
         self.last_tape = None
+        self._fdef: Optional[ast.FunctionDef] = None
+        self._plan: Optional[_Plan] = None
+        self._plannable = True      # False once a walk succeeded that cannot be kept: the next calls do not try again
 
     def __call__(self, *args):
         st = None if _state["plan_only"] else _runtime()[1]     # None: lower only
-        w = _Walker(self.fn, args)
+        if self._fdef is None:
+            self._fdef = _parse(self.fn)
+        plan = self._plan
+        if plan is not None:
+            p = plan.instance(self.fn, self._fdef, args)
+            if p is not None:
+                self.last_plan, self.last_params = plan.text, p
+                self._launch_escape(st, plan.field, p)
+                return
+        self._plan = None
+        if self._plannable:
+            try:
+                self._walk(_Walker(self.fn, self._fdef, args, _Reads()), st)
+                return
+            except (_Depends, LangError):
+                pass        # walked again with the arguments' values, which also says what is wrong where something is
+        self._walk(_Walker(self.fn, self._fdef, args), st)
+        self._plannable = False
+
+    def _walk(self, w: _Walker, st):
         body = [s for s in w.fdef.body if not (isinstance(s, ast.Expr) and isinstance(s.value, ast.Constant))]
         if len(body) != 1 or not isinstance(body[0], ast.For):
             raise LangError("a kernel body must be one struct-for over a field")
@@ -458,7 +647,16 @@ class Kernel:
         if any(isinstance(s, ast.While) for s in stmts):
             self._escape(w, st, target_field, names, stmts)
         else:
+            if w.reads:
+                raise _Depends()
             self._map(w, st, target_field, names, stmts)
+
+    def _launch_escape(self, st: Optional[Stream], fld: Field, p) -> None:
+        if st is None:
+            return
+        if fld.buffer is None:
+            raise LangError("the field was made under plan_only() and holds no device memory")
+        ops.escape_time(st, fld.buffer, p)
 
     # -- escape-time shape -----------------------------------------------------------------------
     def _escape(self, w: _Walker, st: Stream, fld: Field, names, stmts):
@@ -535,7 +733,9 @@ class Kernel:
             raise LangError("the loop body is not the quadratic map z*z + c")
         if cvec is None:
             raise LangError("no constant vector c found")
-        c = cvec[1]
+        # an argument may be a whole component of c: its value here, and the way to compute it in the next call
+        constant = [x.of if isinstance(x, _Uniform) else None for x in cvec[1].c]
+        c = Vector([x.value if isinstance(x, _Uniform) else x for x in cvec[1].c])
         n_idx = 2
         aff_z = [_affine(z0[0], n_idx), _affine(z0[1], n_idx)]
         aff_c = [_affine(c[0], n_idx), _affine(c[1], n_idx)]
@@ -583,11 +783,9 @@ class Kernel:
                               color_scale=scale, transposed=transposed, independent_of=_state["independent_of"])
         self.last_plan = f"escape_time kind={'julia' if kind == L.JULIA else 'mandelbrot'} {cols}x{rows} transposed={transposed}"
         self.last_params = p
-        if st is None:
-            return
-        if fld.buffer is None:
-            raise LangError("the field was made under plan_only() and holds no device memory")
-        ops.escape_time(st, fld.buffer, p)
+        if w.reads:
+            self._plan = _Plan(w.reads, fld, p, constant, self.last_plan)
+        self._launch_escape(st, fld, p)
 
     # -- elementwise shape -----------------------------------------------------------------------
     def _map(self, w: _Walker, st: Stream, fld: Field, names, stmts):
