@@ -1,12 +1,17 @@
 // Row reductions, softmax and column sums of a row-major [rows][cols] float matrix, sm_100a.
 //
-// HBM-bound.  Fast path (cols % 4 == 0 and cols <= 4096): ONE WARP PER ROW, the whole row held
-// in registers (up to 32 float4 per lane), so the row is read from HBM exactly once even for
-// softmax, every load of a row is in flight at once, and the reductions need warp shuffles only
-// (no shared memory, no block barrier).  Any other shape takes a block-per-row kernel that
-// re-reads the row through L1/L2.  Summation order is fixed, so results are bit-reproducible.
+// HBM-bound: every kernel reads a row from HBM once, holds what it needs of it in registers and keeps many 16-byte loads in
+// flight.  Rows whose length is no multiple of 8 start anywhere in a 32-byte sector; their kernels (EDGE) split a row into
+// up to three elements in front of the first 16-byte boundary, float4 groups, and up to three elements behind them, so
+// every length runs at the speed of the round ones.  By row length:
+//   up to 64               a few lanes per row, single elements (row_narrow_kernel)
+//   sums and maxima        a warp, four warps or a block per row, streaming (row_reduce_kernel)
+//   softmax up to 10240    one to 16 warps per row, the row in registers (row_group_kernel)
+//   softmax up to 32768    a block per row, the next row already on its way (row_stream_kernel)
+//   softmax beyond         a block per row, which reads it a second time out of L2 (row_two_pass_kernel)
+// Summation order depends on the shape only, so results are bit-reproducible.
 // The reference project has no counterpart for these operators.
-#include <cfloat>
+#include <atomic>
 #include <cstring>
 
 #include "vrhi_internal.h"
@@ -23,63 +28,163 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+__device__ __forceinline__ float sum4(float4 v) { return (v.x + v.y) + (v.z + v.w); }
+__device__ __forceinline__ float max4(float4 v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
+__device__ __forceinline__ float4 splat4(float v) { return make_float4(v, v, v, v); }
 
 enum { ROW_SUM = 1, ROW_MAX = 2, ROW_SOFTMAX = 4 };
 
-// NV = float4 groups per lane (row length <= NV*128 floats).  WHAT = bit set of outputs.
-template <int NV, int WHAT>
-__global__ void __launch_bounds__(256) row_warp_kernel(const float4 *__restrict__ in, float *__restrict__ out_sum,
-                                                       float *__restrict__ out_max, float4 *__restrict__ out_soft,
-                                                       uint64_t rows, uint32_t cols4) {
+// Where the float4 groups of a row lie.  `first` is the index of the row's first element in an array that starts on a
+// 16-byte boundary.  Thread t < head + tail holds the single element edge(t).  Thread t of T takes the groups
+// t - shift, t - shift + T, ...: `shift` counts the groups between the row's first one and the 128-byte boundary before
+// it, so that a warp's accesses start on a line whatever the row's start.  With shift = 0 every warp of an odd
+// row writes two half sectors (softmax of [4099,10007]: 66 us, and 52 us with the shift).
+template <bool EDGE>
+struct RowParts {
+  uint32_t head, n4, tail, shift;
+  __device__ __forceinline__ RowParts(uint64_t first, uint32_t cols) {
+    head = EDGE ? min((4u - (uint32_t)(first & 3u)) & 3u, cols) : 0u;
+    n4 = (cols - head) >> 2;
+    tail = EDGE ? cols - head - 4u * n4 : 0u;
+    shift = EDGE ? ((uint32_t)(first + head) >> 2) & 7u : 0u;
+  }
+  __device__ __forceinline__ bool has_edge(uint32_t t) const { return EDGE && t < head + tail; }
+  __device__ __forceinline__ uint32_t edge(uint32_t t) const { return t < head ? t : 4u * n4 + t; }
+};
+
+// Partial results of a row's warps: red[0..warps) -> every thread, in warp order (up to 8) or as a tree.
+template <int WARPS, bool MAX>
+__device__ __forceinline__ float combine_warps(const float *red) {
+  if (WARPS <= 8) {
+    float r = red[0];
+#pragma unroll
+    for (int j = 1; j < WARPS; ++j) r = MAX ? fmaxf(r, red[j]) : r + red[j];
+    return r;
+  }
   const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t r = warp; r < rows; r += n_warps) {
-    const float4 *src = in + r * cols4;
-    float4 v[NV];
+  const float r = lane < (uint32_t)WARPS ? red[lane] : (MAX ? -INFINITY : 0.f);
+  return MAX ? warp_max(r) : warp_sum(r);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Sums or maxima: TPR threads per row, ROWS rows per group of threads at a time, U float4 in flight per thread and row.
+// Against a block of 256 threads per row with single-element loads and a barrier per row (the path of every odd
+// length before) and a warp per row that held up to 4096 elements in registers.
+template <int TPR, int ROWS, int U, bool MAX, bool EDGE>
+__global__ void __launch_bounds__(TPR > 256 ? TPR : 256) row_reduce_kernel(const float *__restrict__ in, float *__restrict__ out,
+                                                                           uint64_t rows, uint64_t cols) {
+  constexpr int THREADS = TPR > 256 ? TPR : 256, GROUPS = THREADS / TPR, WARPS = TPR / 32;
+  constexpr float ID = MAX ? -INFINITY : 0.f;
+  __shared__ float red[THREADS / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, group = threadIdx.x / TPR, t = threadIdx.x % TPR;
+  const uint64_t most4 = cols >> 2, per_block = (uint64_t)GROUPS * ROWS;
+  for (uint64_t base = (uint64_t)blockIdx.x * per_block; base < rows; base += (uint64_t)gridDim.x * per_block) {
+    const uint64_t r0 = base + (uint64_t)group * ROWS;
+    float acc[ROWS];
+    const float4 *src4[ROWS];
+    uint64_t n4[ROWS];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      const uint32_t c = lane + 32u * k;
-      // lanes past the row end hold the identity of both reductions' inputs
-      v[k] = (c < cols4) ? __ldcs(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < ROWS; ++q) {
+      const bool active = r0 + q < rows;
+      const uint64_t first = (r0 + q) * cols;
+      const uint32_t head = EDGE ? (4u - (uint32_t)(first & 3u)) & 3u : 0u;  // cols > 64 here
+      n4[q] = active ? (cols - head) >> 2 : 0;
+      src4[q] = reinterpret_cast<const float4 *>(in + first + head);
+      acc[q] = ID;
+      if constexpr (EDGE) {
+        const uint32_t tail = (uint32_t)((cols - head) & 3u);
+        if (active && t < head + tail) acc[q] = __ldcs(in + first + (t < head ? t : 4u * n4[q] + t));
+      }
     }
-    float s = 0.f, m = -FLT_MAX;
-    if (WHAT & ROW_SUM) {
+    for (uint64_t c0 = 0; c0 < most4; c0 += (uint64_t)TPR * U) {
+      float4 v[ROWS][U];
 #pragma unroll
-      for (int k = 0; k < NV; ++k) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
-      s = warp_sum(s);
+      for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+          const uint64_t c = c0 + t + (uint32_t)(TPR * k);
+          v[q][k] = c < n4[q] ? __ldcs(src4[q] + c) : splat4(ID);
+        }
+#pragma unroll
+      for (int q = 0; q < ROWS; ++q) {
+        float p[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) p[k] = MAX ? max4(v[q][k]) : sum4(v[q][k]);
+#pragma unroll
+        for (int n = U / 2; n > 0; n >>= 1)
+#pragma unroll
+          for (int k = 0; k < n; ++k) p[k] = MAX ? fmaxf(p[k], p[k + n]) : p[k] + p[k + n];
+        acc[q] = MAX ? fmaxf(acc[q], p[0]) : acc[q] + p[0];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      float r = MAX ? warp_max(acc[q]) : warp_sum(acc[q]);
+      if (WARPS > 1) {  // ROWS is 1 here
+        if (lane == 0) red[warp] = r;
+        __syncthreads();
+        r = combine_warps<WARPS, MAX>(red + group * WARPS);
+        __syncthreads();
+      }
+      if (t == 0 && r0 + q < rows) out[r0 + q] = r;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Rows of at most L * V elements: L lanes per row, V elements per lane, lane j those at j, j + L, ...  A warp's rows are
+// adjacent, so its loads cover one contiguous range.  One warp per row would leave most lanes without an element.
+template <int L, int V, int WHAT>
+__global__ void __launch_bounds__(256) row_narrow_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
+                                                         float *__restrict__ out_max, float *__restrict__ out_soft,
+                                                         uint64_t rows, uint32_t cols) {
+  constexpr uint32_t FULL = 0xffffffffu;
+  const uint32_t j = threadIdx.x % L;
+  constexpr uint64_t per_block = 256 / L;
+  for (uint64_t base = (uint64_t)blockIdx.x * per_block; base < rows; base += (uint64_t)gridDim.x * per_block) {
+    const uint64_t r = base + threadIdx.x / L;
+    const bool active = r < rows;
+    const float *src = in + r * cols;
+    float x[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) x[k] = active && j + L * k < cols ? __ldg(src + j + L * k) : 0.f;
+    if (WHAT & ROW_SUM) {
+      float s[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) s[k] = x[k];
+#pragma unroll
+      for (int n = V / 2; n > 0; n >>= 1)
+#pragma unroll
+        for (int k = 0; k < n; ++k) s[k] += s[k + n];
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) s[0] += __shfl_xor_sync(FULL, s[0], o);
+      if (active && j == 0) out_sum[r] = s[0];
     }
     if (WHAT & (ROW_MAX | ROW_SOFTMAX)) {
-      float mm = -INFINITY;
+      float m = -INFINITY;
 #pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const uint32_t c = lane + 32u * k;
-        if (c < cols4) mm = fmaxf(mm, fmaxf(fmaxf(v[k].x, v[k].y), fmaxf(v[k].z, v[k].w)));
-      }
-      m = warp_max(mm);
-    }
-    if (lane == 0) {
-      if (WHAT & ROW_SUM) out_sum[r] = s;
-      if (WHAT & ROW_MAX) out_max[r] = m;
-    }
-    if (WHAT & ROW_SOFTMAX) {
-      float z = 0.f;
+      for (int k = 0; k < V; ++k)
+        if (j + L * k < cols) m = fmaxf(m, x[k]);
 #pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const uint32_t c = lane + 32u * k;
-        if (c < cols4) {
-          v[k].x = expf(v[k].x - m); v[k].y = expf(v[k].y - m);
-          v[k].z = expf(v[k].z - m); v[k].w = expf(v[k].w - m);
-          z += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+      for (int o = L / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+      if ((WHAT & ROW_MAX) && active && j == 0) out_max[r] = m;
+      if (WHAT & ROW_SOFTMAX) {
+        float z[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          x[k] = j + L * k < cols ? expf(x[k] - m) : 0.f;
+          z[k] = x[k];
         }
-      }
-      z = warp_sum(z);
-      const float inv = 1.0f / z;
-      float4 *dst = out_soft + r * cols4;
 #pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const uint32_t c = lane + 32u * k;
-        if (c < cols4) __stcs(dst + c, make_float4(v[k].x * inv, v[k].y * inv, v[k].z * inv, v[k].w * inv));
+        for (int n = V / 2; n > 0; n >>= 1)
+#pragma unroll
+          for (int k = 0; k < n; ++k) z[k] += z[k + n];
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) z[0] += __shfl_xor_sync(FULL, z[0], o);
+        const float inv = 1.0f / z[0];
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+          if (active && j + L * k < cols) out_soft[r * cols + j + L * k] = x[k] * inv;
       }
     }
   }
@@ -94,40 +199,54 @@ __device__ __forceinline__ float exp2_approx(float t) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
   return r;
 }
+// Rows of an odd length and of more than 8192 elements take expf: HBM-bound all the same, and more accurate for elements
+// far below the maximum.
+template <bool EXPF>
+struct RowExp {
+  float m, ml;
+  __device__ __forceinline__ explicit RowExp(float max) : m(max), ml(-max * 1.4426950408889634f) {}
+  __device__ __forceinline__ float operator()(float x) const {
+    return EXPF ? expf(x - m) : exp2_approx(fmaf(x, 1.4426950408889634f, ml));
+  }
+  __device__ __forceinline__ float4 operator()(float4 v) const { return make_float4((*this)(v.x), (*this)(v.y), (*this)(v.z), (*this)(v.w)); }
+};
 
 // Softmax rows: WPR warps share one row (8 float4 per thread at most), so a 256-thread CTA works
 // on 8/WPR rows at a time with ~64 registers per thread and 32 resident warps per SM: enough
 // independent warps to keep loads in flight while others are in their exp phase.  The row still
 // makes exactly one trip from HBM and one back.  Cross-warp reductions go through three separate
-// shared arrays (sum, max, normaliser), one CTA barrier each; partials are combined in warp
+// shared arrays (sum, max, normaliser), one CTA barrier each; partials are combined in a fixed
 // order, so results do not depend on scheduling.
-template <int NV, int WPR, int WHAT>
-__global__ void __launch_bounds__(256) row_group_kernel(const float4 *__restrict__ in, float *__restrict__ out_sum,
-                                                        float *__restrict__ out_max, float4 *__restrict__ out_soft,
-                                                        uint64_t rows, uint32_t cols4) {
-  constexpr int GROUPS = 8 / WPR;
+template <int NV, int WPR, int WHAT, bool EDGE>
+__global__ void __launch_bounds__(WPR > 8 ? 32 * WPR : 256, WPR > 8 ? 3 : WPR > 4 ? 5 : 4) row_group_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
+                                                                           float *__restrict__ out_max, float *__restrict__ out_soft,
+                                                                           uint64_t rows, uint32_t cols) {
+  constexpr int GROUPS = WPR > 8 ? 1 : 8 / WPR;
   constexpr uint32_t TPR = 32u * WPR;  // threads per row
-  __shared__ float red_sum[8], red_max[8], red_z[8];
+  __shared__ float red_sum[GROUPS * WPR], red_max[GROUPS * WPR], red_z[GROUPS * WPR];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t group = warp / WPR, wig = warp % WPR;
-  const uint32_t t = wig * 32u + lane;
-  const float kLog2e = 1.4426950408889634f;
+  const uint32_t group = warp / WPR, t = threadIdx.x % TPR;
   for (uint64_t base = (uint64_t)blockIdx.x * GROUPS; base < rows; base += (uint64_t)gridDim.x * GROUPS) {
-    const uint64_t r = base + group;
+    const uint64_t r = base + group, first = r * cols;
     const bool active = r < rows;
-    const float4 *src = in + r * cols4;
+    const RowParts<EDGE> parts(first, cols);
+    const float4 *src = reinterpret_cast<const float4 *>(in + first + parts.head);
+    const uint32_t n4 = parts.n4;
+    const bool has_edge = active && parts.has_edge(t);
     float4 v[NV];
+    float e = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const uint32_t c = t + TPR * k;
-      v[k] = (active && c < cols4) ? __ldcs(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const uint32_t c = t + TPR * k - parts.shift;  // below the row: wraps above n4
+      v[k] = (active && c < n4) ? __ldcs(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float s = 0.f, mm = -INFINITY;
+    if (EDGE && has_edge) e = __ldcs(in + first + parts.edge(t));
+    float s = e, mm = EDGE && has_edge ? e : -INFINITY;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const uint32_t c = t + TPR * k;
-      if (WHAT & ROW_SUM) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
-      if (c < cols4) mm = fmaxf(mm, fmaxf(fmaxf(v[k].x, v[k].y), fmaxf(v[k].z, v[k].w)));
+      const uint32_t c = t + TPR * k - parts.shift;  // below the row: wraps above n4
+      if (WHAT & ROW_SUM) s += sum4(v[k]);
+      if (c < n4) mm = fmaxf(mm, max4(v[k]));
     }
     if (WHAT & ROW_SUM) s = warp_sum(s);
     mm = warp_max(mm);
@@ -137,145 +256,326 @@ __global__ void __launch_bounds__(256) row_group_kernel(const float4 *__restrict
         red_max[warp] = mm;
       }
       __syncthreads();
-      s = 0.f; mm = -INFINITY;
+      if (WPR <= 8) {
+        s = 0.f; mm = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < WPR; ++j) {
-        if (WHAT & ROW_SUM) s += red_sum[group * WPR + j];
-        mm = fmaxf(mm, red_max[group * WPR + j]);
+        for (int j = 0; j < WPR; ++j) {
+          if (WHAT & ROW_SUM) s += red_sum[group * WPR + j];
+          mm = fmaxf(mm, red_max[group * WPR + j]);
+        }
+      } else
+      {
+      if (WHAT & ROW_SUM) s = combine_warps<WPR, false>(red_sum + group * WPR);
+      mm = combine_warps<WPR, true>(red_max + group * WPR);
       }
     }
     if (active && t == 0) {
       if (WHAT & ROW_SUM) out_sum[r] = s;
       if (WHAT & ROW_MAX) out_max[r] = mm;
     }
-    if (WHAT & ROW_SOFTMAX) {
-      const float ml = -mm * kLog2e;
-      float z = 0.f;
+    const RowExp<(EDGE || WPR > 8)> ex(mm);
+    float z = 0.f;
+    if (EDGE && has_edge) { e = ex(e); z = e; }
 #pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const uint32_t c = t + TPR * k;
-        if (c < cols4) {
-          v[k].x = exp2_approx(fmaf(v[k].x, kLog2e, ml)); v[k].y = exp2_approx(fmaf(v[k].y, kLog2e, ml));
-          v[k].z = exp2_approx(fmaf(v[k].z, kLog2e, ml)); v[k].w = exp2_approx(fmaf(v[k].w, kLog2e, ml));
-          z += (v[k].x + v[k].y) + (v[k].z + v[k].w);
-        }
+    for (int k = 0; k < NV; ++k) {
+      const uint32_t c = t + TPR * k - parts.shift;  // below the row: wraps above n4
+      if (c < n4) {
+        v[k] = ex(v[k]);
+        z += sum4(v[k]);
       }
-      z = warp_sum(z);
-      if (WPR > 1) {
-        if (lane == 0) red_z[warp] = z;
-        __syncthreads();
+    }
+    z = warp_sum(z);
+    if (WPR > 1) {
+      if (lane == 0) red_z[warp] = z;
+      __syncthreads();
+      if (WPR <= 8) {
         z = 0.f;
 #pragma unroll
         for (int j = 0; j < WPR; ++j) z += red_z[group * WPR + j];
-      }
-      const float inv = 1.0f / z;
-      float4 *dst = out_soft + r * cols4;
+      } else
+      z = combine_warps<WPR, false>(red_z + group * WPR);
+    }
+    const float inv = 1.0f / z;
+    float4 *dst = reinterpret_cast<float4 *>(out_soft + first + parts.head);
 #pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const uint32_t c = t + TPR * k;
-        if (active && c < cols4) __stcs(dst + c, make_float4(v[k].x * inv, v[k].y * inv, v[k].z * inv, v[k].w * inv));
+    for (int k = 0; k < NV; ++k) {
+      const uint32_t c = t + TPR * k - parts.shift;  // below the row: wraps above n4
+      if (active && c < n4) __stcs(dst + c, make_float4(v[k].x * inv, v[k].y * inv, v[k].z * inv, v[k].w * inv));
+    }
+    if (EDGE && has_edge) __stcs(out_soft + first + parts.edge(t), e * inv);
+  }
+}
+
+// Softmax of longer rows: a resident grid whose blocks go from row to row, the next row on its way into shared memory
+// (cp.async, each thread its own 16-byte slots) while this one is in registers.  A block per row as above needs three
+// or more blocks per SM that happen to be in different phases; a row of 64 KiB leaves room for two, and they wait for
+// their loads together: [4000,16384] 116 us, 135 us for [2048,32768], where the row is all of the SM's registers.
+__device__ __forceinline__ void cp_async_16(void *smem_dst, const void *gmem_src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
+}
+
+template <int T, int NV, int WHAT, bool EDGE>
+__global__ void __launch_bounds__(T, 1024 / T) row_stream_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
+                                                                 float *__restrict__ out_max, float *__restrict__ out_soft,
+                                                                 uint64_t rows, uint32_t cols) {
+  constexpr int WARPS = T / 32;
+  extern __shared__ float4 stage[];  // [NV][T]: slot k of thread t is stage[k * T + t], written and read by that thread only
+  // A row's uses of each array lie between two barriers that the next row's uses are behind, so one copy is enough.
+  __shared__ float red_sum[WARPS], red_max[WARPS], red_z[WARPS];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  float e_next = 0.f;
+  auto fetch = [&](uint64_t r) {
+    if (r < rows) {
+      const uint64_t first = r * cols;
+      const RowParts<EDGE> parts(first, cols);
+      const float4 *src = reinterpret_cast<const float4 *>(in + first + parts.head);
+      const uint32_t c0 = t - parts.shift;  // groups in front of the row wrap above n4
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (c0 + T * k < parts.n4) cp_async_16(stage + k * T + t, src + (c0 + T * k));
+      if (parts.has_edge(t)) e_next = __ldcs(in + first + parts.edge(t));
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint64_t r = blockIdx.x;
+  fetch(r);
+  for (; r < rows; r += gridDim.x) {
+    const uint64_t first = r * cols;
+    const RowParts<EDGE> parts(first, cols);
+    const uint32_t c0 = t - parts.shift, n4 = parts.n4;
+    const bool has_edge = parts.has_edge(t);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float4 v[NV];
+    float e = has_edge ? e_next : 0.f;
+    float s = e, mm = has_edge ? e : -INFINITY;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c0 + T * k < n4) {
+        v[k] = stage[k * T + t];
+        mm = fmaxf(mm, max4(v[k]));
+        if (WHAT & ROW_SUM) s += sum4(v[k]);
       }
     }
+    if (WHAT & ROW_SUM) s = warp_sum(s);
+    mm = warp_max(mm);
+    if (lane == 0) {
+      if (WHAT & ROW_SUM) red_sum[warp] = s;
+      red_max[warp] = mm;
+    }
+    __syncthreads();
+    fetch(r + gridDim.x);  // behind the barrier: the slots have been read
+    if (WHAT & ROW_SUM) s = combine_warps<WARPS, false>(red_sum);
+    mm = combine_warps<WARPS, true>(red_max);
+    if (t == 0) {
+      if (WHAT & ROW_SUM) out_sum[r] = s;
+      if (WHAT & ROW_MAX) out_max[r] = mm;
+    }
+    const RowExp<(EDGE || T > 256)> ex(mm);
+    float z = 0.f;
+    if (has_edge) { e = ex(e); z = e; }
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (c0 + T * k < n4) {
+        v[k] = ex(v[k]);
+        z += sum4(v[k]);
+      }
+    z = warp_sum(z);
+    if (lane == 0) red_z[warp] = z;
+    __syncthreads();
+    z = combine_warps<WARPS, false>(red_z);
+    const float inv = 1.0f / z;
+    float4 *dst = reinterpret_cast<float4 *>(out_soft + first + parts.head);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (c0 + T * k < n4) __stcs(dst + (c0 + T * k), make_float4(v[k].x * inv, v[k].y * inv, v[k].z * inv, v[k].w * inv));
+    if (has_edge) __stcs(out_soft + first + parts.edge(t), e * inv);
   }
 }
 
-// Any shape: one 256-thread block per row, scalar accesses, three passes for softmax.
-__device__ __forceinline__ float block_reduce(float v, bool is_max, float *smem) {
-  v = is_max ? warp_max(v) : warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();  // smem reuse across consecutive calls
-  if (l == 0) smem[w] = v;
-  __syncthreads();
-  float r = (l < 8) ? smem[l] : (is_max ? -INFINITY : 0.f);
-  r = is_max ? warp_max(r) : warp_sum(r);
-  return r;
-}
-
-template <int WHAT>
-__global__ void __launch_bounds__(256) row_block_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
-                                                        float *__restrict__ out_max, float *__restrict__ out_soft,
-                                                        uint64_t rows, uint64_t cols) {
-  __shared__ float smem[8];
+// Softmax of rows that a block's registers do not hold: two passes, the second one out of L2 (two rows per SM under way:
+// 296 rows of 65536 elements are 78 MB of the 126).  The first pass keeps a running maximum per thread and the sum of the
+// exponentials relative to it, so the row is read twice and not three times.
+template <int WHAT, bool EDGE>
+__global__ void __launch_bounds__(512, 3) row_two_pass_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
+                                                              float *__restrict__ out_max, float *__restrict__ out_soft,
+                                                              uint64_t rows, uint64_t cols) {
+  constexpr uint32_t T = 512, U = 4, WARPS = T / 32;
+  __shared__ float red_sum[WARPS], red_max[WARPS], red_z[WARPS];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
   for (uint64_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const float *src = in + r * cols;
-    float s = 0.f, m = -INFINITY;
-    for (uint64_t c = threadIdx.x; c < cols; c += 256) {
-      float x = src[c];
-      s += x;
-      m = fmaxf(m, x);
+    const uint64_t first = r * cols;
+    const uint32_t head = EDGE ? (4u - (uint32_t)(first & 3u)) & 3u : 0u;
+    const uint64_t n4 = (cols - head) >> 2, edges = head + ((cols - head) & 3u), shift = EDGE ? ((first + head) >> 2) & 7u : 0u;
+    const bool has_edge = t < edges;
+    const uint64_t at = first + (t < head ? t : 4u * n4 + t);
+    const float4 *src = reinterpret_cast<const float4 *>(in + first + head);
+    float e = has_edge ? __ldg(in + at) : 0.f;
+    float s = e, m = has_edge ? e : -INFINITY, z = has_edge ? 1.f : 0.f;
+    if (has_edge && e != e) z = e;  // a NaN is not its own maximum
+    for (uint64_t c0 = 0; c0 < n4 + shift; c0 += T * U) {
+      float4 v[U];
+      float chunk = -INFINITY;
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) {
+        const uint64_t c = c0 + t + T * k - shift;
+        v[k] = splat4(-INFINITY);
+        if (c < n4) v[k] = __ldg(src + c);
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) {
+        chunk = fmaxf(chunk, max4(v[k]));
+        if (WHAT & ROW_SUM) s += c0 + t + T * k - shift < n4 ? sum4(v[k]) : 0.f;
+      }
+      const float next = fmaxf(m, chunk);
+      // next = -inf: nothing but -inf (and NaN) so far; such a row's results are NaN through the second pass unless more follows
+      if (next > m) { z *= expf(m - next); m = next; }
+      const float ref = m == -INFINITY ? 0.f : m;
+      float p[U];
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) p[k] = sum4(make_float4(expf(v[k].x - ref), expf(v[k].y - ref), expf(v[k].z - ref), expf(v[k].w - ref)));
+#pragma unroll
+      for (uint32_t n = U / 2; n > 0; n >>= 1)
+#pragma unroll
+        for (uint32_t k = 0; k < n; ++k) p[k] += p[k + n];
+      z += p[0];
     }
-    if (WHAT & ROW_SUM) {
-      s = block_reduce(s, false, smem);
-      if (threadIdx.x == 0) out_sum[r] = s;
+    if (WHAT & ROW_SUM) s = warp_sum(s);
+    float mm = warp_max(m);
+    if (lane == 0) {
+      if (WHAT & ROW_SUM) red_sum[warp] = s;
+      red_max[warp] = mm;
     }
-    if (WHAT & (ROW_MAX | ROW_SOFTMAX)) {
-      m = block_reduce(m, true, smem);
-      if ((WHAT & ROW_MAX) && threadIdx.x == 0) out_max[r] = m;
+    __syncthreads();
+    if (WHAT & ROW_SUM) s = combine_warps<WARPS, false>(red_sum);
+    mm = combine_warps<WARPS, true>(red_max);
+    if (t == 0) {
+      if (WHAT & ROW_SUM) out_sum[r] = s;
+      if (WHAT & ROW_MAX) out_max[r] = mm;
     }
-    if (WHAT & ROW_SOFTMAX) {
-      float z = 0.f;
-      for (uint64_t c = threadIdx.x; c < cols; c += 256) z += expf(src[c] - m);
-      z = block_reduce(z, false, smem);
-      const float inv = 1.0f / z;
-      float *dst = out_soft + r * cols;
-      for (uint64_t c = threadIdx.x; c < cols; c += 256) dst[c] = expf(src[c] - m) * inv;
+    z = m == mm ? z : z * expf(m - mm);  // (m = mm = +inf would be inf - inf)
+    z = warp_sum(z);
+    if (lane == 0) red_z[warp] = z;
+    __syncthreads();
+    z = combine_warps<WARPS, false>(red_z);
+    const float inv = 1.0f / z;
+    const RowExp<true> ex(mm);
+    float4 *dst = reinterpret_cast<float4 *>(out_soft + first + head);
+    for (uint64_t c0 = 0; c0 < n4 + shift; c0 += T * U) {
+      float4 v[U];
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) {
+        const uint64_t c = c0 + t + T * k - shift;
+        if (c < n4) v[k] = __ldcs(src + c);
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) {
+        const uint64_t c = c0 + t + T * k - shift;
+        if (c >= n4) continue;
+        const float4 y = ex(v[k]);
+        __stcs(dst + c, make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv));
+      }
     }
+    if (has_edge) __stcs(out_soft + at, ex(e) * inv);
   }
+}
+
+static unsigned row_grid(uint64_t rows, uint64_t per_block) {
+  const uint64_t want = (rows + per_block - 1) / per_block;
+  return (unsigned)(want < 0x7fffffffull ? want : 0x7fffffffull);
+}
+
+template <bool MAX, bool EDGE>
+static void launch_reduce(cudaStream_t s, const float *in, float *out, uint64_t rows, uint64_t cols) {
+  if (cols <= 256) row_reduce_kernel<32, 4, 2, MAX, EDGE><<<row_grid(rows, 32), 256, 0, s>>>(in, out, rows, cols);
+  else if (cols <= 1024) row_reduce_kernel<32, 1, 8, MAX, EDGE><<<row_grid(rows, 8), 256, 0, s>>>(in, out, rows, cols);
+  else if (cols <= 4096) row_reduce_kernel<128, 1, 8, MAX, EDGE><<<row_grid(rows, 2), 256, 0, s>>>(in, out, rows, cols);
+  else if (cols <= 16384) row_reduce_kernel<256, 1, 8, MAX, EDGE><<<row_grid(rows, 1), 256, 0, s>>>(in, out, rows, cols);
+  else row_reduce_kernel<1024, 1, 8, MAX, EDGE><<<row_grid(rows, 1), 1024, 0, s>>>(in, out, rows, cols);
+}
+
+template <int T, int NV, int WHAT, bool EDGE>
+static cudaError_t launch_stream_nv(vrhi_stream_t *st, const float *in, float *osum, float *omax, float *osoft, uint64_t rows, uint32_t cols) {
+  auto kern = row_stream_kernel<T, NV, WHAT, EDGE>;
+  constexpr int smem = NV * T * (int)sizeof(float4);
+  static std::atomic<uint64_t> raised{0};  // devices on which the kernel's shared memory limit has been raised (always to the same value)
+  const uint64_t bit = 1ull << (st->dev->ordinal & 63);
+  if (!(raised.load(std::memory_order_acquire) & bit)) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    raised.fetch_or(bit, std::memory_order_release);
+  }
+  const uint64_t resident = (uint64_t)st->dev->prop.multiProcessorCount * (1024 / T);
+  kern<<<(unsigned)(rows < resident ? rows : resident), T, smem, st->s>>>(in, osum, omax, osoft, rows, cols);
+  return cudaGetLastError();
+}
+
+template <int T, int WHAT, bool EDGE>
+static cudaError_t launch_stream(vrhi_stream_t *st, const float *in, float *osum, float *omax, float *osoft, uint64_t rows, uint32_t cols, uint64_t most4) {
+  const uint64_t nv = (most4 + T - 1) / T;
+  if (nv <= 5) return launch_stream_nv<T, 5, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
+  if (nv <= 6) return launch_stream_nv<T, 6, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
+  if (nv <= 7) return launch_stream_nv<T, 7, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
+  return launch_stream_nv<T, 8, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
+}
+
+template <int WHAT, bool EDGE>
+static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osum, float *omax, float *osoft, uint64_t rows, uint64_t cols) {
+  cudaStream_t s = st->s;
+  const uint64_t most4 = cols / 4 + (EDGE ? 7 : 0);  // with the groups in front of a row (RowParts::shift)
+  if (most4 > 8192) {
+    const uint64_t resident = (uint64_t)st->dev->prop.multiProcessorCount * 3;
+    row_two_pass_kernel<WHAT, EDGE><<<(unsigned)(rows < resident ? rows : resident), 512, 0, s>>>(in, osum, omax, osoft, rows, cols);
+    return cudaGetLastError();
+  }
+  if (most4 > 4096) return launch_stream<1024, WHAT, EDGE>(st, in, osum, omax, osoft, rows, (uint32_t)cols, most4);
+  if (most4 > 2560) return launch_stream<512, WHAT, EDGE>(st, in, osum, omax, osoft, rows, (uint32_t)cols, most4);
+  // Registers for a row of the block's: 64 per thread with 8 float4 (four blocks of 256 threads per SM), 40 with 5 (three of 512,
+  // six of 256).  One more block per SM in another phase is worth more than any other choice here: [4096,10000] 50.7 us
+  // with three blocks of 512 threads per SM, 60 us with two.
+  const uint32_t wpr = most4 <= 256 ? 1 : most4 <= 512 ? 2 : most4 <= 1024 ? 4 : most4 <= 1280 ? 8 : 16;
+  const uint32_t nv = (uint32_t)((most4 + 32u * wpr - 1) / (32u * wpr));
+  // one CTA per group of rows, not a persistent grid: measured on B200, letting the hardware
+  // scheduler stream CTAs (each loads, reduces, writes and leaves) beats a resident grid whose
+  // CTAs fall into lock step, all loading and then all storing (0.314 ms against 0.36 ms on [65536,4096])
+  const unsigned grid = row_grid(rows, wpr > 8 ? 1 : 8 / wpr), block = wpr > 8 ? 32 * wpr : 256;
+#define GROUP_LAUNCH(NV, WPR) row_group_kernel<NV, WPR, WHAT, EDGE><<<grid, block, 0, s>>>(in, osum, omax, osoft, rows, (uint32_t)cols)
+#define GROUP_NV(WPR)                     \
+  do {                                    \
+    if (nv <= 5) GROUP_LAUNCH(5, WPR);    \
+    else if (nv <= 6) GROUP_LAUNCH(6, WPR); \
+    else GROUP_LAUNCH(8, WPR);            \
+  } while (0)
+  if (wpr == 1) {
+    if (nv <= 1) GROUP_LAUNCH(1, 1);
+    else if (nv <= 2) GROUP_LAUNCH(2, 1);
+    else if (nv <= 4) GROUP_LAUNCH(4, 1);
+    else GROUP_LAUNCH(8, 1);
+  } else if (wpr == 2) GROUP_NV(2);
+  else if (wpr == 4) GROUP_NV(4);
+  else if (wpr == 8) GROUP_LAUNCH(5, 8);
+  else if (nv <= 3) GROUP_LAUNCH(3, 16);
+  else if (nv <= 4) GROUP_LAUNCH(4, 16);
+  else GROUP_LAUNCH(5, 16);
+#undef GROUP_NV
+#undef GROUP_LAUNCH
+  return cudaGetLastError();
 }
 
 template <int WHAT>
 static int launch_rows(vrhi_stream_t *st, const float *in, float *osum, float *omax, float *osoft, uint64_t rows, uint64_t cols,
                        const char *name) {
-  const int sms = st->dev->prop.multiProcessorCount;
-  if ((WHAT & ROW_SOFTMAX) && cols % 4 == 0 && cols <= 8192) {
-    const uint32_t cols4 = (uint32_t)(cols / 4);
-    const float4 *i4 = (const float4 *)in;
-    float4 *o4 = (float4 *)osoft;
-    const int wpr = cols4 <= 256 ? 1 : cols4 <= 512 ? 2 : cols4 <= 1024 ? 4 : 8;
-    const uint32_t nv = (cols4 + 32u * wpr - 1) / (32u * wpr);
-    const uint64_t groups = 8 / wpr;
-    uint64_t want = (rows + groups - 1) / groups;
-    // one CTA per group of rows, not a persistent grid: measured on B200, letting the hardware
-    // scheduler stream CTAs (each loads, reduces, writes and leaves) beats a resident grid whose
-    // CTAs fall into lock step, all loading and then all storing (0.314 ms against 0.36 ms on [65536,4096])
-    uint64_t cap = 0x7fffffffull;
-    unsigned grid = (unsigned)(want < cap ? want : cap);
-#define GROUP_LAUNCH(NV, WPR) row_group_kernel<NV, WPR, (WHAT | ROW_SOFTMAX)><<<grid, 256, 0, st->s>>>(i4, osum, omax, o4, rows, cols4)
-#define GROUP_NV(WPR)                 \
-  do {                                \
-    if (nv <= 1) GROUP_LAUNCH(1, WPR); \
-    else if (nv <= 2) GROUP_LAUNCH(2, WPR); \
-    else if (nv <= 4) GROUP_LAUNCH(4, WPR); \
-    else GROUP_LAUNCH(8, WPR);        \
-  } while (0)
-    if (wpr == 1) GROUP_NV(1);
-    else if (wpr == 2) GROUP_NV(2);
-    else if (wpr == 4) GROUP_NV(4);
-    else GROUP_NV(8);
-#undef GROUP_NV
-#undef GROUP_LAUNCH
-  } else if (cols % 4 == 0 && cols <= 4096) {
-    const uint32_t cols4 = (uint32_t)(cols / 4);
-    const uint32_t nv = (cols4 + 31) / 32;
-    // softmax keeps the row live across two reductions: fewer resident warps, so more CTAs of
-    // rows in flight do not help; 8 warps per CTA, CTAs = min(rows/8, SMs * 8)
-    uint64_t want = (rows + 7) / 8;
-    uint64_t cap = (uint64_t)sms * 8;
-    unsigned grid = (unsigned)(want < cap ? want : cap);
-    const float4 *i4 = (const float4 *)in;
-    float4 *o4 = (float4 *)osoft;
-#define ROWS_LAUNCH(NV) row_warp_kernel<NV, WHAT><<<grid, 256, 0, st->s>>>(i4, osum, omax, o4, rows, cols4)
-    if (nv <= 1) ROWS_LAUNCH(1);
-    else if (nv <= 2) ROWS_LAUNCH(2);
-    else if (nv <= 4) ROWS_LAUNCH(4);
-    else if (nv <= 8) ROWS_LAUNCH(8);
-    else if (nv <= 16) ROWS_LAUNCH(16);
-    else ROWS_LAUNCH(32);
-#undef ROWS_LAUNCH
+  if (cols <= 16) row_narrow_kernel<4, 4, WHAT><<<row_grid(rows, 64), 256, 0, st->s>>>(in, osum, omax, osoft, rows, (uint32_t)cols);
+  else if (cols <= 64) row_narrow_kernel<8, 8, WHAT><<<row_grid(rows, 32), 256, 0, st->s>>>(in, osum, omax, osoft, rows, (uint32_t)cols);
+  else if constexpr ((WHAT & ROW_SOFTMAX) != 0) {
+    VRHI_CUDA((cols % 8 != 0 ? launch_softmax<WHAT, true>(st, in, osum, omax, osoft, rows, cols)  // rows that start inside a 32-byte sector
+                             : launch_softmax<WHAT, false>(st, in, osum, omax, osoft, rows, cols)));
   } else {
-    uint64_t cap = (uint64_t)sms * 8;
-    unsigned grid = (unsigned)(rows < cap ? rows : cap);
-    row_block_kernel<WHAT><<<grid, 256, 0, st->s>>>(in, osum, omax, osoft, rows, cols);
+    constexpr bool MAX = WHAT == ROW_MAX;
+    float *out = MAX ? omax : osum;
+    if (cols % 4 != 0) launch_reduce<MAX, true>(st->s, in, out, rows, cols);
+    else launch_reduce<MAX, false>(st->s, in, out, rows, cols);
   }
   return post_launch(st, name);
 }
