@@ -17,7 +17,7 @@
 
 namespace vrhi {
 
-struct Mat4 {
+struct __align__(16) Mat4 {
   float m[16];  // row-major
 };
 
@@ -30,28 +30,59 @@ __device__ __forceinline__ float4 matvec4(const Mat4 &M, float4 v) {
   return r;
 }
 
-__global__ void __launch_bounds__(256) vertex_transform_kernel(const float *__restrict__ pos, const float *__restrict__ model,
+// A block takes 1024 vertices: their positions, one contiguous range, come in as float4s, go out again as the varying
+// in the same registers, and lie in shared memory while every thread transforms four vertices (stride 3 words: no bank
+// conflicts).  All global accesses are 16 bytes per thread and contiguous per warp.  Measured on B200, 1000003 vertices:
+// 7.9 us with a thread per vertex (4-byte accesses, 12 bytes apart; a last wave of a third of the blocks), 6.4 us so; 2^24: 161 and 109 us.
+constexpr int kVerts = 1024;
+__global__ void __launch_bounds__(256, 4) vertex_transform_kernel(const float *__restrict__ pos, const float *__restrict__ model,
                                                                const float *__restrict__ view, const float *__restrict__ proj,
                                                                float4 *__restrict__ out_pos, float *__restrict__ out_varying,
                                                                uint64_t n) {
+  __shared__ __align__(16) float tile[3 * kVerts];
   __shared__ Mat4 sm[3];
-  if (threadIdx.x < 48) {
-    const float *src = threadIdx.x < 16 ? model : (threadIdx.x < 32 ? view : proj);
-    sm[threadIdx.x / 16].m[threadIdx.x % 16] = src[threadIdx.x % 16];
+  const uint32_t t = threadIdx.x;
+  if (t < 48) {
+    const float *src = t < 16 ? model : (t < 32 ? view : proj);
+    sm[t / 16].m[t % 16] = src[t % 16];
   }
-  __syncthreads();
-  const Mat4 Mm = sm[0], Mv = sm[1], Mp = sm[2];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
-    const float p0 = pos[3 * k], p1 = pos[3 * k + 1], p2 = pos[3 * k + 2];
-    float4 v = make_float4(p0, p1, p2, 1.0f);
-    v = matvec4(Mm, v);
-    v = matvec4(Mv, v);
-    v = matvec4(Mp, v);
-    __stcs(out_pos + k, v);
-    out_varying[3 * k] = p0;
-    out_varying[3 * k + 1] = p1;
-    out_varying[3 * k + 2] = p2;
+  for (uint64_t base = (uint64_t)blockIdx.x * kVerts; base < n; base += (uint64_t)gridDim.x * kVerts) {
+    const uint32_t here = (uint32_t)(n - base < kVerts ? n - base : kVerts), floats = 3 * here;
+    const float4 *src4 = reinterpret_cast<const float4 *>(pos + 3 * base);
+    float4 *var4 = reinterpret_cast<float4 *>(out_varying + 3 * base);
+    float4 v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (4 * (t + 256 * k) + 3 < floats) v[k] = __ldcs(src4 + t + 256 * k);
+    const uint32_t left = floats & ~3u;  // the up to three floats behind the last float4
+    const float edge = t < (floats & 3u) ? pos[3 * base + left + t] : 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (4 * (t + 256 * k) + 3 < floats) {
+        __stcs(var4 + t + 256 * k, v[k]);
+        reinterpret_cast<float4 *>(tile)[t + 256 * k] = v[k];
+      }
+    if (t < (floats & 3u)) {
+      out_varying[3 * base + left + t] = edge;
+      tile[left + t] = edge;
+    }
+    __syncthreads();
+    float4 p[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t k = t + 256 * q;
+      p[q] = k < here ? make_float4(tile[3 * k], tile[3 * k + 1], tile[3 * k + 2], 1.0f) : make_float4(0.f, 0.f, 0.f, 1.0f);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const Mat4 M = sm[m];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) p[q] = matvec4(M, p[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (t + 256 * q < here) __stcs(out_pos + base + t + 256 * q, p[q]);
+    __syncthreads();  // the tile may be filled again
   }
 }
 
@@ -76,7 +107,7 @@ int launch_vertex_transform(vrhi_stream_t *st, const ArgView *args, int n_args, 
   for (int k = 0; k < 6; ++k)
     if (args[k].bytes < need[k]) return fail(VRHI_ERR_SIZE, "vertex_transform: argument %d holds %llu bytes, %llu needed", k, (unsigned long long)args[k].bytes, (unsigned long long)need[k]);
   if (!writable(args[4]) || !writable(args[5])) return fail(VRHI_ERR_INVALID, "vertex_transform: an output buffer is read-only");
-  vertex_transform_kernel<<<grid_for(st, q.n), 256, 0, st->s>>>((const float *)args[0].ptr, (const float *)args[1].ptr, (const float *)args[2].ptr,
+  vertex_transform_kernel<<<grid_for(st, (q.n + 3) / 4), 256, 0, st->s>>>((const float *)args[0].ptr, (const float *)args[1].ptr, (const float *)args[2].ptr,
                                                                 (const float *)args[3].ptr, (float4 *)args[4].ptr, (float *)args[5].ptr, q.n);
   return post_launch(st, "vertex_transform");
 }
