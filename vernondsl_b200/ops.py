@@ -7,6 +7,7 @@ computes: a missing library or an unsupported shape raises.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Optional, Sequence
 
 import numpy as np
@@ -40,6 +41,26 @@ def op_names() -> list:
 def launch(stream: Stream, name: str, args: Sequence[L.Arg], params) -> None:
     arr = (L.Arg * len(args))(*args)
     check(lib().vrhi_op_launch(stream._h, op_id(name), arr, len(args), C.byref(params), C.sizeof(params)))
+
+
+# The operators below lay their arguments and parameter blocks out with struct, one call each: filling the ctypes structures
+# field by field took longer than the kernels of small problems (vertex_transform: 12 us per call, its kernel 6).
+_ARG = "QQQii"                       # vrhi_arg: buffer, offset, bytes, class, reserved
+_ARGS = [struct.Struct(_ARG * n) for n in range(17)]
+_ROWS, _MAP, _MSE = struct.Struct("IIQQ"), struct.Struct("IIQ"), struct.Struct("IIQQd")
+_M64 = (1 << 64) - 1                 # as ctypes converts: modulo 2^64
+
+
+def _launch(stream: Stream, name: str, args: Sequence, params, params_size: int) -> None:
+    """``args``: (buffer, class) pairs, whole buffers."""
+    fields = []
+    for b, cls in args:
+        h = b._h
+        fields += (h.value if h else 0, 0, 0, cls, 0)
+    n = len(args)
+    rc = lib().vrhi_op_launch(stream._h, _op_ids[name] if name in _op_ids else op_id(name), (_ARGS[n] if n < 17 else struct.Struct(_ARG * n)).pack(*fields), n, params, params_size)
+    if rc:
+        check(rc)
 
 
 # ------------------------------------------------------------------------------ escape time ---
@@ -77,12 +98,12 @@ def escape_time(stream: Stream, image: Buffer, params: L.EscapeParams, wire: Opt
     """Launch the escape-time map (the per-pixel loop of fractal.py:18-25) into ``image``.  ``wire``,
     a uint16 image of the same geometry, receives every count a second time (the form sent to peers);
     ``byte_plane`` (with ``wire``), a uint8 plane, receives min(count, 255)."""
-    args = [image.arg(L.IMAGE if image.arg_class == L.IMAGE else L.OUTPUT)]
+    args = [(image, L.IMAGE if image.arg_class == L.IMAGE else L.OUTPUT)]
     if wire is not None:
-        args.append(wire.arg(L.IMAGE if wire.arg_class == L.IMAGE else L.OUTPUT))
+        args.append((wire, L.IMAGE if wire.arg_class == L.IMAGE else L.OUTPUT))
         if byte_plane is not None:
-            args.append(byte_plane.arg(L.IMAGE if byte_plane.arg_class == L.IMAGE else L.OUTPUT))
-    launch(stream, "escape_time", args, params)
+            args.append((byte_plane, L.IMAGE if byte_plane.arg_class == L.IMAGE else L.OUTPUT))
+    _launch(stream, "escape_time", args, C.byref(params), C.sizeof(params))
 
 
 def widen_rows_u16(stream: Stream, wire: Buffer, image: Buffer, width: int, height: int, chunk_rows: int, world: int,
@@ -131,9 +152,7 @@ def gather_pull_u16(stream: Stream, flags: Buffer, image: Buffer, peer_wires: Se
 # ------------------------------------------------------------------------------ maps ----------
 def fused_map(stream: Stream, a: Buffer, x: Buffer, y: Buffer, out: Buffer, n: int) -> None:
     """out = tanh(a*x + y) * exp(-0.5*x*x) + sqrt(|y| + 1e-3), one kernel."""
-    p = L.MapParams()
-    p.size, p.n = C.sizeof(L.MapParams), int(n)
-    launch(stream, "fused_map", [a.arg(L.INPUT), x.arg(L.INPUT), y.arg(L.INPUT), out.arg(L.OUTPUT)], p)
+    _launch(stream, "fused_map", ((a, L.INPUT), (x, L.INPUT), (y, L.INPUT), (out, L.OUTPUT)), _MAP.pack(16, 0, int(n) & _M64), 16)
 
 
 class Tape:
@@ -188,16 +207,35 @@ class Tape:
             p.instr[k].op, p.instr[k].a, p.instr[k].b, p.instr[k].c, p.instr[k].imm = op, a, b, c, imm
         return p
 
+    _HEAD, _TAIL, _INSTR = struct.Struct("IIIIQQIII%dI" % L.TAPE_MAX_OUTPUTS), struct.Struct("III"), struct.Struct("HHHHf")
+
+    def _block(self, rows: int, cols: int, flags: int) -> bytes:
+        """``params`` as bytes, laid out directly."""
+        n_instr, n_out = len(self.instr), len(self.outputs)
+        if n_instr > L.TAPE_MAX_INSTR or n_out > L.TAPE_MAX_OUTPUTS or self.n_inputs > L.TAPE_MAX_INPUTS:
+            raise ValueError("tape exceeds the operator's limits")
+        try:
+            pack = self._INSTR.pack
+            return b"".join([
+                self._HEAD.pack(C.sizeof(L.TapeParams), self.n_inputs, n_out, n_instr, int(rows), int(cols), self.row_mask, self.col_mask,
+                                self.scalar_mask, *self.outputs, *(0,) * (L.TAPE_MAX_OUTPUTS - n_out)),
+                *[pack(*i) for i in self.instr], bytes(self._INSTR.size * (L.TAPE_MAX_INSTR - n_instr)),
+                self._TAIL.pack(flags, getattr(self, "colsum_mask", 0), 0), bytes(self._END)])
+        except (struct.error, OverflowError):   # numbers that ctypes converts and struct refuses
+            p = self.params(rows, cols)
+            p.flags |= flags
+            return bytes(p)
+
+    _END = C.sizeof(L.TapeParams) - _HEAD.size - _INSTR.size * L.TAPE_MAX_INSTR - _TAIL.size
+
 
 def map_tape(stream: Stream, tape: Tape, inputs: Sequence[Buffer], outputs: Sequence[Buffer], rows: int, cols: int,
              interpret: bool = False) -> None:
     """Run the tape over [rows][cols] arrays as one kernel: compiled for this tape at first use, or, with
     ``interpret`` (and where no run-time compiler is installed), by the interpreting kernel.  Same bits either way."""
-    args = [b.arg(L.INPUT) for b in inputs] + [b.arg(L.OUTPUT) for b in outputs]
-    p = tape.params(rows, cols)
-    if interpret:
-        p.flags |= L.TAPE_FLAG_INTERPRET
-    launch(stream, "map_tape", args, p)
+    p = tape._block(rows, cols, L.TAPE_FLAG_INTERPRET if interpret else 0)
+    args = [(b, L.INPUT) for b in inputs] + [(b, L.OUTPUT) for b in outputs]
+    _launch(stream, "map_tape", args, p, len(p))
 
 
 def tape_jit_stats() -> dict:
@@ -218,33 +256,30 @@ def tape_source(tape: Tape, rows: int = 4, cols: int = 4) -> str:
 
 
 # ------------------------------------------------------------------------------ rows ----------
-def _rows(rows: int, cols: int) -> L.RowsParams:
-    p = L.RowsParams()
-    p.size, p.rows, p.cols = C.sizeof(L.RowsParams), int(rows), int(cols)
-    return p
+def _rows(rows: int, cols: int) -> bytes:
+    return _ROWS.pack(24, 0, int(rows) & _M64, int(cols) & _M64)
 
 
 def row_sum(stream: Stream, m: Buffer, out: Buffer, rows: int, cols: int) -> None:
-    launch(stream, "row_sum", [m.arg(L.INPUT), out.arg(L.OUTPUT)], _rows(rows, cols))
+    _launch(stream, "row_sum", ((m, L.INPUT), (out, L.OUTPUT)), _rows(rows, cols), 24)
 
 
 def row_max(stream: Stream, m: Buffer, out: Buffer, rows: int, cols: int) -> None:
-    launch(stream, "row_max", [m.arg(L.INPUT), out.arg(L.OUTPUT)], _rows(rows, cols))
+    _launch(stream, "row_max", ((m, L.INPUT), (out, L.OUTPUT)), _rows(rows, cols), 24)
 
 
 def row_softmax(stream: Stream, m: Buffer, out: Buffer, rows: int, cols: int) -> None:
-    launch(stream, "row_softmax", [m.arg(L.INPUT), out.arg(L.OUTPUT)], _rows(rows, cols))
+    _launch(stream, "row_softmax", ((m, L.INPUT), (out, L.OUTPUT)), _rows(rows, cols), 24)
 
 
 def row_stats_softmax(stream: Stream, m: Buffer, out_sum: Buffer, out_max: Buffer, out_softmax: Buffer, rows: int,
                       cols: int) -> None:
     """Per-row sum, per-row max and softmax(row) from a single read of the matrix."""
-    launch(stream, "row_stats_softmax",
-           [m.arg(L.INPUT), out_sum.arg(L.OUTPUT), out_max.arg(L.OUTPUT), out_softmax.arg(L.OUTPUT)], _rows(rows, cols))
+    _launch(stream, "row_stats_softmax", ((m, L.INPUT), (out_sum, L.OUTPUT), (out_max, L.OUTPUT), (out_softmax, L.OUTPUT)), _rows(rows, cols), 24)
 
 
 def col_sum(stream: Stream, m: Buffer, out: Buffer, rows: int, cols: int) -> None:
-    launch(stream, "col_sum", [m.arg(L.INPUT), out.arg(L.OUTPUT)], _rows(rows, cols))
+    _launch(stream, "col_sum", ((m, L.INPUT), (out, L.OUTPUT)), _rows(rows, cols), 24)
 
 
 # ------------------------------------------------------------------------------ loss / grad ---
@@ -257,34 +292,29 @@ def _mse(rows: int, cols: int, denom: float) -> L.MseParams:
 def mse_tanh_fwd(stream: Stream, W: Buffer, x: Buffer, b: Buffer, t: Buffer, loss: Buffer, rows: int, cols: int,
                  denom: float = 0.0) -> None:
     """loss = sum((tanh(W*x + b) - t)^2) / denom over these rows (denom = 0: rows*cols)."""
-    launch(stream, "mse_tanh_fwd", [W.arg(L.INPUT), x.arg(L.INPUT), b.arg(L.INPUT), t.arg(L.INPUT), loss.arg(L.OUTPUT)],
-           _mse(rows, cols, denom))
+    _launch(stream, "mse_tanh_fwd", ((W, L.INPUT), (x, L.INPUT), (b, L.INPUT), (t, L.INPUT), (loss, L.OUTPUT)),
+            _MSE.pack(32, 0, int(rows) & _M64, int(cols) & _M64, denom), 32)
 
 
 def mse_tanh_bwd(stream: Stream, W: Buffer, x: Buffer, b: Buffer, t: Buffer, dW: Buffer, dx: Buffer, db: Buffer,
                  rows: int, cols: int, denom: float = 0.0, loss: Optional[Buffer] = None) -> None:
     """dW, dx (full size) and db (column sums) of the loss above, forward recomputed in the kernel."""
-    args = [W.arg(L.INPUT), x.arg(L.INPUT), b.arg(L.INPUT), t.arg(L.INPUT), dW.arg(L.OUTPUT), dx.arg(L.OUTPUT),
-            db.arg(L.OUTPUT)]
+    args = [(W, L.INPUT), (x, L.INPUT), (b, L.INPUT), (t, L.INPUT), (dW, L.OUTPUT), (dx, L.OUTPUT), (db, L.OUTPUT)]
     if loss is not None:
-        args.append(loss.arg(L.OUTPUT))
-    launch(stream, "mse_tanh_bwd", args, _mse(rows, cols, denom))
+        args.append((loss, L.OUTPUT))
+    _launch(stream, "mse_tanh_bwd", args, _MSE.pack(32, 0, int(rows) & _M64, int(cols) & _M64, denom), 32)
 
 
 def vertex_transform(stream: Stream, pos: Buffer, model: Buffer, view: Buffer, proj: Buffer, gl_position: Buffer,
                      varying: Buffer, n: int) -> None:
     """color.mlir:4-39 over an array of n vertices: gl_position = proj*(view*(model*(p,1))), varying = p."""
-    p = L.MapParams()
-    p.size, p.n = C.sizeof(L.MapParams), int(n)
-    launch(stream, "vertex_transform", [pos.arg(L.INPUT), model.arg(L.UNIFORM), view.arg(L.UNIFORM), proj.arg(L.UNIFORM),
-                                        gl_position.arg(L.OUTPUT), varying.arg(L.VARYING)], p)
+    _launch(stream, "vertex_transform", ((pos, L.INPUT), (model, L.UNIFORM), (view, L.UNIFORM), (proj, L.UNIFORM), (gl_position, L.OUTPUT),
+                                         (varying, L.VARYING)), _MAP.pack(16, 0, int(n) & _M64), 16)
 
 
 def flat_color(stream: Stream, color: Buffer, fragments: Buffer, n: int) -> None:
     """color.mlir:43-59 over n fragments: every fragment = (c0, c1, c2, 1)."""
-    p = L.MapParams()
-    p.size, p.n = C.sizeof(L.MapParams), int(n)
-    launch(stream, "flat_color", [color.arg(L.UNIFORM), fragments.arg(L.IMAGE)], p)
+    _launch(stream, "flat_color", ((color, L.UNIFORM), (fragments, L.IMAGE)), _MAP.pack(16, 0, int(n) & _M64), 16)
 
 
 def fp32_probe(stream: Stream, out: Buffer, ffma_per_thread: int, threads: int = 0, variant: int = 0) -> None:
