@@ -31,6 +31,8 @@ struct EscapeDev {
   uint32_t n_batches;
   uint32_t transposed;       // 1: the row coordinate is the real part and the column coordinate the imaginary part
   float neg_zero;            // -0.0f, set by the host: an addend the assembler cannot fold (k_escape_pair.cu)
+  uint32_t ordered;          // 1: everything before the launch has to have finished when it begins (begin_launch)
+  uint32_t chained;          // host: the launch carries the programmatic-serialization attribute
   uint8_t *bytes;            // optional third copy of every count, min(count, 255), at the same pixel index (nullptr: none)
 };
 
@@ -165,14 +167,18 @@ __device__ __forceinline__ uint32_t escape_count(float zr, float zi, float cr, f
   return count;
 }
 
-// A launch that its caller declared independent of the launches before it is started with the
-// programmatic-serialization attribute: its blocks may become resident as soon as every block of the
-// launch before it has passed begin_overlap(), i.e. at once, beside that launch's blocks.  Every
-// block calls end_overlap() last: the grid then cannot complete before the grid before it has, so
-// whatever follows on the stream in the ordinary way still finds everything earlier finished.
-// Both are no-ops in a launch without the attribute and nothing after it that carries it.
-__device__ __forceinline__ void begin_overlap() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void end_overlap() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The blocks of a launch that carries the programmatic-serialization attribute (EscapeDev::chained) may become resident
+// as soon as every block of the launch before it has executed launch_dependents.  An ordinary launch waits in
+// begin_launch() until everything before it has finished, and only then lets the next one come.  A launch that its caller
+// declared independent of the launches before it does not wait there and runs beside them; every block ends with
+// end_launch(), so its grid cannot complete before the grid before it has, and whatever follows on the stream still
+// finds everything earlier finished.  (Were the next launch let in before the wait, one that is independent of this
+// launch, but not of what came before it, could start too early.)  All of it is a no-op without the attribute.
+__device__ __forceinline__ void begin_launch(const EscapeDev &p) {
+  if (p.ordered) asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void end_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Work stealing: the next batch for this warp, n_batches or more when none is left.  A launch makes exactly n_batches
 // fetches that succeed and one that fails per warp, so the wrapping increment leaves the counter at 0 behind the
@@ -181,22 +187,6 @@ __device__ __forceinline__ void end_overlap() { asm volatile("griddepcontrol.wai
 // The host keeps n_batches + warps within 32 bits.
 __device__ __forceinline__ uint32_t next_batch(uint32_t *counter, uint32_t n_batches) {
   return atomicInc(counter, n_batches + gridDim.x * (blockDim.x >> 5) - 1u);
-}
-
-// Launch `kern` on the stream; `overlap`: with the attribute described above.
-template <class Kern, class... Args>
-cudaError_t launch_maybe_overlapped(Kern kern, int grid, int block, size_t dyn, cudaStream_t s, bool overlap, Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = dyn;
-  cfg.stream = s;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = overlap ? 1u : 0u;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // Order in which a launch visits its rows: from the middle outwards (k = 0 is the middle row).  The
@@ -228,7 +218,7 @@ __device__ __forceinline__ uint32_t owned_row_to_image_row(const EscapeDev &p, u
 // launches from several host threads never see a limit below what they ask for.
 template <class Kern>
 int launch_pinned(Kern kern, int grid, int per_sm, vrhi_stream_t *st, const EscapeDev &p, void *image, uint32_t *counter,
-                  uint16_t *wire, bool pin = true, bool overlap = false) {
+                  uint16_t *wire, bool pin = true) {
   struct Entry { size_t fixed; size_t limit; };
   static std::mutex mu;
   static std::unordered_map<uint64_t, Entry> cache;  // key: kernel address mixed with the device ordinal
@@ -255,16 +245,15 @@ int launch_pinned(Kern kern, int grid, int per_sm, vrhi_stream_t *st, const Esca
       it->second.limit = dyn;
     }
   }
-  if (overlap) VRHI_CUDA(launch_maybe_overlapped(kern, grid, 256, dyn, st->s, true, p, image, counter, wire));
-  else kern<<<grid, 256, dyn, st->s>>>(p, image, counter, wire);
+  VRHI_CUDA(launch_chained(p.chained, kern, dim3((unsigned)grid), 256, dyn, st->s, p, image, counter, wire));
   return VRHI_OK;
 }
 
 // the regrouping kernel (k_escape_pair.cu); it needs max_iter >= 12, the length of its blocks and of its intake
-int launch_escape_pair(vrhi_stream_t *st, const vrhi_escape_params &q, const EscapeDev &p, int grid, int per_sm, bool pin, bool overlap,
+int launch_escape_pair(vrhi_stream_t *st, const vrhi_escape_params &q, const EscapeDev &p, int grid, int per_sm, bool pin,
                        void *image, uint32_t *counter, uint16_t *wire);
 
 // the kernel for launches with little to regroup (k_escape_block.cu)
-int launch_escape_block(vrhi_stream_t *st, const vrhi_escape_params &q, EscapeDev p, bool overlap, void *image, uint16_t *wire);
+int launch_escape_block(vrhi_stream_t *st, const vrhi_escape_params &q, EscapeDev p, void *image, uint16_t *wire);
 
 }  // namespace vrhi

@@ -29,7 +29,7 @@ namespace vrhi {
 template <int KIND, int MODE, int OUT>
 __global__ void __launch_bounds__(256) escape_checked_kernel(EscapeDev p, void *image, uint32_t *work_counter, uint16_t *wire) {
   const uint32_t lane = threadIdx.x & 31u;
-  begin_overlap();
+  begin_launch(p);
   // work_counter == nullptr: batches are dealt to warps round-robin (small frames, where the
   // counter's reset would cost as much as the frame); otherwise warps pull batches from the counter
   uint32_t next = blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -63,16 +63,16 @@ __global__ void __launch_bounds__(256) escape_checked_kernel(EscapeDev p, void *
       if (wire) store_wire(wire, p.bytes, row_base + i, count);
     }
   }
-  end_overlap();
+  end_launch();
 }
 
 template <int KIND, int MODE>
-static void launch_checked(int out, int grid, cudaStream_t s, bool overlap, const EscapeDev &p, void *image, uint32_t *ctr, uint16_t *wire) {
+static void launch_checked(int out, int grid, cudaStream_t s, const EscapeDev &p, void *image, uint32_t *ctr, uint16_t *wire) {
   uint16_t *const none = nullptr;
   switch (out) {
-    case VRHI_OUT_COUNT_U32: launch_maybe_overlapped(escape_checked_kernel<KIND, MODE, VRHI_OUT_COUNT_U32>, grid, 256, 0, s, overlap, p, image, ctr, wire); break;
-    case VRHI_OUT_COUNT_U16: launch_maybe_overlapped(escape_checked_kernel<KIND, MODE, VRHI_OUT_COUNT_U16>, grid, 256, 0, s, overlap, p, image, ctr, none); break;
-    default: launch_maybe_overlapped(escape_checked_kernel<KIND, MODE, VRHI_OUT_COLOR_F32>, grid, 256, 0, s, overlap, p, image, ctr, none); break;
+    case VRHI_OUT_COUNT_U32: launch_chained(p.chained, escape_checked_kernel<KIND, MODE, VRHI_OUT_COUNT_U32>, dim3((unsigned)grid), 256, 0, s, p, image, ctr, wire); break;
+    case VRHI_OUT_COUNT_U16: launch_chained(p.chained, escape_checked_kernel<KIND, MODE, VRHI_OUT_COUNT_U16>, dim3((unsigned)grid), 256, 0, s, p, image, ctr, none); break;
+    default: launch_chained(p.chained, escape_checked_kernel<KIND, MODE, VRHI_OUT_COLOR_F32>, dim3((unsigned)grid), 256, 0, s, p, image, ctr, none); break;
   }
 }
 
@@ -189,9 +189,11 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
   const uint32_t independent_of = (q.flags & VRHI_ESCAPE_FLAG_INDEPENDENT_MASK) >> VRHI_ESCAPE_FLAG_INDEPENDENT_SHIFT;
   const int run = st->escape_chain;  // launches of the current run so far
   const bool overlap = independent_of != 0 && run >= 1 && (uint32_t)run <= independent_of && run < 8;
+  p.ordered = overlap ? 0u : 1u;
+  p.chained = overlap || chains(st) ? 1u : 0u;
   const int run_after = independent_of == 0 ? 0 : overlap ? run + 1 : 1;
   if (blocks_ok && !regroup_ok && p.rows_owned <= 1u << 31) {
-    VRHI_TRY(launch_escape_block(st, q, p, overlap, args[0].ptr, wire));
+    VRHI_TRY(launch_escape_block(st, q, p, args[0].ptr, wire));
     VRHI_TRY(post_launch(st, "escape_time (blocks)"));
     st->escape_chain = run_after;
     return VRHI_OK;
@@ -252,17 +254,17 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
     // frame's blocks should move in while this frame's last ones drain (65 -> 41 us per 1080p frame
     // with two alternating streams), and a few tens of microseconds cannot go far out of balance.
     const bool pin = per_sm >= 3;
-    VRHI_TRY(launch_escape_pair(st, q, p, grid, (int)per_sm, pin, overlap, args[0].ptr, counter, wire));
+    VRHI_TRY(launch_escape_pair(st, q, p, grid, (int)per_sm, pin, args[0].ptr, counter, wire));
     VRHI_TRY(post_launch(st, "escape_time (two pixels per lane)"));
     st->escape_chain = run_after;
     return VRHI_OK;
   }
   if (q.kind == VRHI_ESCAPE_MANDELBROT) {
-    if (q.mode == VRHI_ESCAPE_EXACT) launch_checked<VRHI_ESCAPE_MANDELBROT, VRHI_ESCAPE_EXACT>(q.output, grid, st->s, overlap, p, args[0].ptr, counter, wire);
-    else launch_checked<VRHI_ESCAPE_MANDELBROT, VRHI_ESCAPE_FAST>(q.output, grid, st->s, overlap, p, args[0].ptr, counter, wire);
+    if (q.mode == VRHI_ESCAPE_EXACT) launch_checked<VRHI_ESCAPE_MANDELBROT, VRHI_ESCAPE_EXACT>(q.output, grid, st->s, p, args[0].ptr, counter, wire);
+    else launch_checked<VRHI_ESCAPE_MANDELBROT, VRHI_ESCAPE_FAST>(q.output, grid, st->s, p, args[0].ptr, counter, wire);
   } else {
-    if (q.mode == VRHI_ESCAPE_EXACT) launch_checked<VRHI_ESCAPE_JULIA, VRHI_ESCAPE_EXACT>(q.output, grid, st->s, overlap, p, args[0].ptr, counter, wire);
-    else launch_checked<VRHI_ESCAPE_JULIA, VRHI_ESCAPE_FAST>(q.output, grid, st->s, overlap, p, args[0].ptr, counter, wire);
+    if (q.mode == VRHI_ESCAPE_EXACT) launch_checked<VRHI_ESCAPE_JULIA, VRHI_ESCAPE_EXACT>(q.output, grid, st->s, p, args[0].ptr, counter, wire);
+    else launch_checked<VRHI_ESCAPE_JULIA, VRHI_ESCAPE_FAST>(q.output, grid, st->s, p, args[0].ptr, counter, wire);
   }
   VRHI_TRY(post_launch(st, "escape_time"));
   st->escape_chain = run_after;

@@ -17,7 +17,7 @@ constexpr uint32_t kTileW = 8, kTileH = 8;
 
 template <int KIND, int OUT, int MODE, bool WIRE, int U>
 __global__ void __launch_bounds__(256) escape_block_kernel(EscapeDev p, void *image, uint16_t *wire) {
-  begin_overlap();
+  begin_launch(p);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t FULL = 0xffffffffu;
   const uint32_t batch = blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -114,26 +114,26 @@ __global__ void __launch_bounds__(256) escape_block_kernel(EscapeDev p, void *im
       }
     }
   }
-  end_overlap();
+  end_launch();
 }
 
 template <int KIND, int OUT, bool WIRE, int U>
-static cudaError_t launch_mode(uint32_t mode, int grid, cudaStream_t s, bool overlap, const EscapeDev &p, void *image, uint16_t *wire) {
-  if (mode == VRHI_ESCAPE_EXACT) return launch_maybe_overlapped(escape_block_kernel<KIND, OUT, VRHI_ESCAPE_EXACT, WIRE, U>, grid, 256, 0, s, overlap, p, image, wire);
-  return launch_maybe_overlapped(escape_block_kernel<KIND, OUT, VRHI_ESCAPE_FAST, WIRE, U>, grid, 256, 0, s, overlap, p, image, wire);
+static cudaError_t launch_mode(uint32_t mode, int grid, cudaStream_t s, const EscapeDev &p, void *image, uint16_t *wire) {
+  if (mode == VRHI_ESCAPE_EXACT) return launch_chained(p.chained, escape_block_kernel<KIND, OUT, VRHI_ESCAPE_EXACT, WIRE, U>, dim3((unsigned)grid), 256, 0, s, p, image, wire);
+  return launch_chained(p.chained, escape_block_kernel<KIND, OUT, VRHI_ESCAPE_FAST, WIRE, U>, dim3((unsigned)grid), 256, 0, s, p, image, wire);
 }
 
 template <int KIND, int U>
-static cudaError_t launch_out(const vrhi_escape_params &q, int grid, cudaStream_t s, bool overlap, const EscapeDev &p, void *image, uint16_t *wire) {
-  if (wire) return launch_mode<KIND, VRHI_OUT_COUNT_U32, true, U>(q.mode, grid, s, overlap, p, image, wire);
+static cudaError_t launch_out(const vrhi_escape_params &q, int grid, cudaStream_t s, const EscapeDev &p, void *image, uint16_t *wire) {
+  if (wire) return launch_mode<KIND, VRHI_OUT_COUNT_U32, true, U>(q.mode, grid, s, p, image, wire);
   switch (q.output) {
-    case VRHI_OUT_COUNT_U32: return launch_mode<KIND, VRHI_OUT_COUNT_U32, false, U>(q.mode, grid, s, overlap, p, image, nullptr);
-    case VRHI_OUT_COUNT_U16: return launch_mode<KIND, VRHI_OUT_COUNT_U16, false, U>(q.mode, grid, s, overlap, p, image, nullptr);
-    default: return launch_mode<KIND, VRHI_OUT_COLOR_F32, false, U>(q.mode, grid, s, overlap, p, image, nullptr);
+    case VRHI_OUT_COUNT_U32: return launch_mode<KIND, VRHI_OUT_COUNT_U32, false, U>(q.mode, grid, s, p, image, nullptr);
+    case VRHI_OUT_COUNT_U16: return launch_mode<KIND, VRHI_OUT_COUNT_U16, false, U>(q.mode, grid, s, p, image, nullptr);
+    default: return launch_mode<KIND, VRHI_OUT_COLOR_F32, false, U>(q.mode, grid, s, p, image, nullptr);
   }
 }
 
-int launch_escape_block(vrhi_stream_t *st, const vrhi_escape_params &q, EscapeDev p, bool overlap, void *image, uint16_t *wire) {
+int launch_escape_block(vrhi_stream_t *st, const vrhi_escape_params &q, EscapeDev p, void *image, uint16_t *wire) {
   p.tiles_per_row = (p.width + kTileW - 1) / kTileW;
   const uint64_t tile_rows = ((uint64_t)p.rows_owned + kTileH - 1) / kTileH, tiles = p.tiles_per_row * tile_rows;
   // Adjacent tiles of a row of tiles per warp, so that a tile's share of the row's index arithmetic is small, as long as
@@ -151,11 +151,11 @@ int launch_escape_block(vrhi_stream_t *st, const vrhi_escape_params &q, EscapeDe
   // 45.2 and 43.3 us; Mandelbrot 50.2 and 47.4).
   const bool shallow = q.max_iter < 128u;
   if (q.kind == VRHI_ESCAPE_MANDELBROT) {
-    if (shallow) VRHI_CUDA((launch_out<VRHI_ESCAPE_MANDELBROT, 4>(q, grid, st->s, overlap, p, image, wire)));
-    else VRHI_CUDA((launch_out<VRHI_ESCAPE_MANDELBROT, 8>(q, grid, st->s, overlap, p, image, wire)));
+    if (shallow) VRHI_CUDA((launch_out<VRHI_ESCAPE_MANDELBROT, 4>(q, grid, st->s, p, image, wire)));
+    else VRHI_CUDA((launch_out<VRHI_ESCAPE_MANDELBROT, 8>(q, grid, st->s, p, image, wire)));
   } else {
-    if (shallow) VRHI_CUDA((launch_out<VRHI_ESCAPE_JULIA, 4>(q, grid, st->s, overlap, p, image, wire)));
-    else VRHI_CUDA((launch_out<VRHI_ESCAPE_JULIA, 8>(q, grid, st->s, overlap, p, image, wire)));
+    if (shallow) VRHI_CUDA((launch_out<VRHI_ESCAPE_JULIA, 4>(q, grid, st->s, p, image, wire)));
+    else VRHI_CUDA((launch_out<VRHI_ESCAPE_JULIA, 8>(q, grid, st->s, p, image, wire)));
   }
   return VRHI_OK;
 }

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) fused_map_kernel(const float4 *__restrict
                                                         const float4 *__restrict__ y, float4 *__restrict__ out,
                                                         uint64_t n4, uint64_t n, const float *a1, const float *x1,
                                                         const float *y1, float *o1) {
+  pdl_begin();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (; k + (UNROLL - 1) * stride < n4; k += UNROLL * stride) {
@@ -85,9 +86,9 @@ int launch_fused_map(vrhi_stream_t *st, const ArgView *args, int n_args, const v
   static const int env_blocks = env_int("VRHI_MAP_BLOCKS_PER_SM", 1, 32, 0);  // tuning aid
   if (env_blocks) cap = (uint64_t)sms * env_blocks;
   unsigned grid = (unsigned)(want < cap ? (want ? want : 1) : cap);
-  fused_map_kernel<2><<<grid, 256, 0, st->s>>>(
-      (const float4 *)args[0].ptr, (const float4 *)args[1].ptr, (const float4 *)args[2].ptr, (float4 *)args[3].ptr, n4, q.n,
-      (const float *)args[0].ptr, (const float *)args[1].ptr, (const float *)args[2].ptr, (float *)args[3].ptr);
+  VRHI_CUDA(launch_chained(chains(st), fused_map_kernel<2>, dim3(grid), 256, 0, st->s, (const float4 *)args[0].ptr, (const float4 *)args[1].ptr,
+                             (const float4 *)args[2].ptr, (float4 *)args[3].ptr, n4, q.n, (const float *)args[0].ptr, (const float *)args[1].ptr,
+                             (const float *)args[2].ptr, (float *)args[3].ptr));
   return post_launch(st, "fused_map");
 }
 

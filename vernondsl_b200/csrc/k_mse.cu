@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256, 5) mse_bwd_kernel(const float *__restrict
                                                       const MseShape q, float inv) {
   __shared__ float4 red[256];
   __shared__ float smem[8];
-  pdl_release();
+  pdl_begin();
   const float4 *__restrict__ w4 = reinterpret_cast<const float4 *>(W_), *__restrict__ x4 = reinterpret_cast<const float4 *>(X_), *__restrict__ t4 = reinterpret_cast<const float4 *>(T_);
   const uint32_t sub = threadIdx.x / q.W, lane = threadIdx.x - sub * q.W;
   const uint64_t gi = (uint64_t)blockIdx.x * q.W + lane;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256) mse_fwd_kernel(const float *__restrict__ 
                                                       const float *__restrict__ B, const float *__restrict__ T_,
                                                       float *__restrict__ loss_partial, const MseShape q) {
   __shared__ float smem[8];
-  pdl_release();
+  pdl_begin();
   const float4 *__restrict__ w4 = reinterpret_cast<const float4 *>(W_), *__restrict__ x4 = reinterpret_cast<const float4 *>(X_), *__restrict__ t4 = reinterpret_cast<const float4 *>(T_);
   const uint32_t sub = threadIdx.x / q.W, lane = threadIdx.x - sub * q.W;
   const uint64_t gi = (uint64_t)blockIdx.x * q.W + lane;
@@ -257,7 +257,7 @@ int launch_mse_tanh_fwd(vrhi_stream_t *st, const ArgView *args, int n_args, cons
   VRHI_TRY(stream_arena(st, n_part * 4, nullptr, &payload));
   dim3 grid(pl.gx, pl.gy);
   const float *W = (const float *)args[0].ptr, *X = (const float *)args[1].ptr, *B = (const float *)args[2].ptr, *T = (const float *)args[3].ptr;
-  mse_fwd_kernel<<<grid, 256, 0, st->s>>>(W, X, B, T, (float *)payload, pl.shape);
+  VRHI_CUDA(launch_chained(chains(st), mse_fwd_kernel, grid, 256, 0, st->s, W, X, B, T, (float *)payload, pl.shape));
   VRHI_TRY(post_launch(st, "mse_tanh_fwd"));
   FinishJobs jobs{};
   add_finish_job(&jobs, (const float *)payload, (float *)args[4].ptr, (uint32_t)n_part, 1, 1.0 / pl.denom);
@@ -285,7 +285,7 @@ int launch_mse_tanh_bwd(vrhi_stream_t *st, const ArgView *args, int n_args, cons
   dim3 grid(pl.gx, pl.gy);
   const float *W = (const float *)args[0].ptr, *X = (const float *)args[1].ptr, *B = (const float *)args[2].ptr, *T = (const float *)args[3].ptr;
   const float inv = (float)(2.0 / pl.denom);
-  mse_bwd_kernel<<<grid, 256, 0, st->s>>>(W, X, B, T, (float *)args[4].ptr, (float *)args[5].ptr, db_partial, loss_partial, pl.shape, inv);
+  VRHI_CUDA(launch_chained(chains(st), mse_bwd_kernel, grid, 256, 0, st->s, W, X, B, T, (float *)args[4].ptr, (float *)args[5].ptr, db_partial, loss_partial, pl.shape, inv));
   VRHI_TRY(post_launch(st, "mse_tanh_bwd"));
   FinishJobs jobs{};
   add_finish_job(&jobs, db_partial, (float *)args[6].ptr, db_rows, pl.cols, 1.0);

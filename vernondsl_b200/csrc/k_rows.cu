@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(TPR > 256 ? TPR : 256) row_reduce_kernel(const
   constexpr int THREADS = TPR > 256 ? TPR : 256, GROUPS = THREADS / TPR, WARPS = TPR / 32;
   constexpr float ID = MAX ? -INFINITY : 0.f;
   __shared__ float red[THREADS / 32];
+  pdl_begin();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, group = threadIdx.x / TPR, t = threadIdx.x % TPR;
   const uint64_t most4 = cols >> 2, per_block = (uint64_t)GROUPS * ROWS;
   for (uint64_t base = (uint64_t)blockIdx.x * per_block; base < rows; base += (uint64_t)gridDim.x * per_block) {
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(256) row_narrow_kernel(const float *__restrict
                                                          float *__restrict__ out_max, float *__restrict__ out_soft,
                                                          uint64_t rows, uint32_t cols) {
   constexpr uint32_t FULL = 0xffffffffu;
+  pdl_begin();
   const uint32_t j = threadIdx.x % L;
   constexpr uint64_t per_block = 256 / L;
   for (uint64_t base = (uint64_t)blockIdx.x * per_block; base < rows; base += (uint64_t)gridDim.x * per_block) {
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(WPR > 8 ? 32 * WPR : 256, WPR > 8 ? 3 : WPR > 
   constexpr uint32_t TPR = 32u * WPR;  // threads per row
   __shared__ float red_sum[GROUPS * WPR], red_max[GROUPS * WPR], red_z[GROUPS * WPR];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  pdl_begin();
   const uint32_t group = warp / WPR, t = threadIdx.x % TPR;
   for (uint64_t base = (uint64_t)blockIdx.x * GROUPS; base < rows; base += (uint64_t)gridDim.x * GROUPS) {
     const uint64_t r = base + group, first = r * cols;
@@ -338,6 +341,7 @@ __global__ void __launch_bounds__(T, 1024 / T) row_stream_kernel(const float *__
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  pdl_begin();
   uint64_t r = blockIdx.x;
   fetch(r);
   for (; r < rows; r += gridDim.x) {
@@ -403,6 +407,7 @@ __global__ void __launch_bounds__(512, 3) row_two_pass_kernel(const float *__res
                                                               uint64_t rows, uint64_t cols) {
   constexpr uint32_t T = 512, U = 4, WARPS = T / 32;
   __shared__ float red_sum[WARPS], red_max[WARPS], red_z[WARPS];
+  pdl_begin();
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
   for (uint64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const uint64_t first = r * cols;
@@ -487,12 +492,12 @@ static unsigned row_grid(uint64_t rows, uint64_t per_block) {
 }
 
 template <bool MAX, bool EDGE>
-static void launch_reduce(cudaStream_t s, const float *in, float *out, uint64_t rows, uint64_t cols) {
-  if (cols <= 256) row_reduce_kernel<32, 4, 2, MAX, EDGE><<<row_grid(rows, 32), 256, 0, s>>>(in, out, rows, cols);
-  else if (cols <= 1024) row_reduce_kernel<32, 1, 8, MAX, EDGE><<<row_grid(rows, 8), 256, 0, s>>>(in, out, rows, cols);
-  else if (cols <= 4096) row_reduce_kernel<128, 1, 8, MAX, EDGE><<<row_grid(rows, 2), 256, 0, s>>>(in, out, rows, cols);
-  else if (cols <= 16384) row_reduce_kernel<256, 1, 8, MAX, EDGE><<<row_grid(rows, 1), 256, 0, s>>>(in, out, rows, cols);
-  else row_reduce_kernel<1024, 1, 8, MAX, EDGE><<<row_grid(rows, 1), 1024, 0, s>>>(in, out, rows, cols);
+static cudaError_t launch_reduce(vrhi_stream_t *st, const float *in, float *out, uint64_t rows, uint64_t cols) {
+  if (cols <= 256) return launch_chained(chains(st), row_reduce_kernel<32, 4, 2, MAX, EDGE>, dim3(row_grid(rows, 32)), 256, 0, st->s, in, out, rows, cols);
+  if (cols <= 1024) return launch_chained(chains(st), row_reduce_kernel<32, 1, 8, MAX, EDGE>, dim3(row_grid(rows, 8)), 256, 0, st->s, in, out, rows, cols);
+  if (cols <= 4096) return launch_chained(chains(st), row_reduce_kernel<128, 1, 8, MAX, EDGE>, dim3(row_grid(rows, 2)), 256, 0, st->s, in, out, rows, cols);
+  if (cols <= 16384) return launch_chained(chains(st), row_reduce_kernel<256, 1, 8, MAX, EDGE>, dim3(row_grid(rows, 1)), 256, 0, st->s, in, out, rows, cols);
+  return launch_chained(chains(st), row_reduce_kernel<1024, 1, 8, MAX, EDGE>, dim3(row_grid(rows, 1)), 1024, 0, st->s, in, out, rows, cols);
 }
 
 template <int T, int NV, int WHAT, bool EDGE>
@@ -507,8 +512,7 @@ static cudaError_t launch_stream_nv(vrhi_stream_t *st, const float *in, float *o
     raised.fetch_or(bit, std::memory_order_release);
   }
   const uint64_t resident = (uint64_t)st->dev->prop.multiProcessorCount * (1024 / T);
-  kern<<<(unsigned)(rows < resident ? rows : resident), T, smem, st->s>>>(in, osum, omax, osoft, rows, cols);
-  return cudaGetLastError();
+  return launch_chained(chains(st), kern, dim3((unsigned)(rows < resident ? rows : resident)), T, smem, st->s, in, osum, omax, osoft, rows, cols);
 }
 
 template <int T, int WHAT, bool EDGE>
@@ -526,8 +530,7 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
   const uint64_t most4 = cols / 4 + (EDGE ? 7 : 0);  // with the groups in front of a row (RowParts::shift)
   if (most4 > 8192) {
     const uint64_t resident = (uint64_t)st->dev->prop.multiProcessorCount * 3;
-    row_two_pass_kernel<WHAT, EDGE><<<(unsigned)(rows < resident ? rows : resident), 512, 0, s>>>(in, osum, omax, osoft, rows, cols);
-    return cudaGetLastError();
+    return launch_chained(chains(st), row_two_pass_kernel<WHAT, EDGE>, dim3((unsigned)(rows < resident ? rows : resident)), 512, 0, s, in, osum, omax, osoft, rows, cols);
   }
   if (most4 > 4096) return launch_stream<1024, WHAT, EDGE>(st, in, osum, omax, osoft, rows, (uint32_t)cols, most4);
   if (most4 > 2560) return launch_stream<512, WHAT, EDGE>(st, in, osum, omax, osoft, rows, (uint32_t)cols, most4);
@@ -540,7 +543,7 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
   // scheduler stream CTAs (each loads, reduces, writes and leaves) beats a resident grid whose
   // CTAs fall into lock step, all loading and then all storing (0.314 ms against 0.36 ms on [65536,4096])
   const unsigned grid = row_grid(rows, wpr > 8 ? 1 : 8 / wpr), block = wpr > 8 ? 32 * wpr : 256;
-#define GROUP_LAUNCH(NV, WPR) row_group_kernel<NV, WPR, WHAT, EDGE><<<grid, block, 0, s>>>(in, osum, omax, osoft, rows, (uint32_t)cols)
+#define GROUP_LAUNCH(NV, WPR) return launch_chained(chains(st), row_group_kernel<NV, WPR, WHAT, EDGE>, dim3(grid), block, 0, s, in, osum, omax, osoft, rows, (uint32_t)cols)
 #define GROUP_NV(WPR)                     \
   do {                                    \
     if (nv <= 5) GROUP_LAUNCH(5, WPR);    \
@@ -560,22 +563,20 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
   else GROUP_LAUNCH(5, 16);
 #undef GROUP_NV
 #undef GROUP_LAUNCH
-  return cudaGetLastError();
 }
 
 template <int WHAT>
 static int launch_rows(vrhi_stream_t *st, const float *in, float *osum, float *omax, float *osoft, uint64_t rows, uint64_t cols,
                        const char *name) {
-  if (cols <= 16) row_narrow_kernel<4, 4, WHAT><<<row_grid(rows, 64), 256, 0, st->s>>>(in, osum, omax, osoft, rows, (uint32_t)cols);
-  else if (cols <= 64) row_narrow_kernel<8, 8, WHAT><<<row_grid(rows, 32), 256, 0, st->s>>>(in, osum, omax, osoft, rows, (uint32_t)cols);
+  if (cols <= 16) VRHI_CUDA(launch_chained(chains(st), row_narrow_kernel<4, 4, WHAT>, dim3(row_grid(rows, 64)), 256, 0, st->s, in, osum, omax, osoft, rows, (uint32_t)cols));
+  else if (cols <= 64) VRHI_CUDA(launch_chained(chains(st), row_narrow_kernel<8, 8, WHAT>, dim3(row_grid(rows, 32)), 256, 0, st->s, in, osum, omax, osoft, rows, (uint32_t)cols));
   else if constexpr ((WHAT & ROW_SOFTMAX) != 0) {
     VRHI_CUDA((cols % 8 != 0 ? launch_softmax<WHAT, true>(st, in, osum, omax, osoft, rows, cols)  // rows that start inside a 32-byte sector
                              : launch_softmax<WHAT, false>(st, in, osum, omax, osoft, rows, cols)));
   } else {
     constexpr bool MAX = WHAT == ROW_MAX;
     float *out = MAX ? omax : osum;
-    if (cols % 4 != 0) launch_reduce<MAX, true>(st->s, in, out, rows, cols);
-    else launch_reduce<MAX, false>(st->s, in, out, rows, cols);
+    VRHI_CUDA((cols % 4 != 0 ? launch_reduce<MAX, true>(st, in, out, rows, cols) : launch_reduce<MAX, false>(st, in, out, rows, cols)));
   }
   return post_launch(st, name);
 }
@@ -660,7 +661,7 @@ __global__ void __launch_bounds__(256, kColBlocksPerSm<VEC>) col_partial_kernel(
                                                           uint64_t groups, uint32_t W, uint32_t R) {
   typedef typename ColValue<VEC>::type V;
   __shared__ V red[256];
-  pdl_release();
+  pdl_begin();
   const V *__restrict__ in = static_cast<const V *>(in_raw);
   const uint32_t sub = threadIdx.x / W, w = threadIdx.x - sub * W;
   const uint64_t g = (uint64_t)blockIdx.x * W + w;
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(1024) finish_partials_kernel(const __grid_cons
   const uint32_t sub = threadIdx.x / W, w = threadIdx.x - sub * W;
   const uint64_t c = (uint64_t)block * W + w;
   const bool active = sub < R && c < cols;
-  pdl_wait();
+  pdl_begin();
   double s = 0.0;
   if (active) {
     uint32_t g = sub;
@@ -778,11 +779,9 @@ static ColPlan plan_col_sum(uint64_t rows, uint64_t cols, int sms, uint64_t most
 }
 
 // dst: p.gy partial rows, or, where the plan has one block row, the result itself
-static cudaError_t launch_col_partial(cudaStream_t s, const ColPlan &p, const float *in, float *dst, uint64_t rows) {
+static cudaError_t launch_col_partial(bool chain, cudaStream_t s, const ColPlan &p, const float *in, float *dst, uint64_t rows) {
   const dim3 grid(p.gx, p.gy);
-  if (p.vec) col_partial_kernel<true><<<grid, 256, 0, s>>>(in, dst, rows, p.groups, p.W, p.R);
-  else col_partial_kernel<false><<<grid, 256, 0, s>>>(in, dst, rows, p.groups, p.W, p.R);
-  return cudaGetLastError();
+  return launch_chained(chain, p.vec ? col_partial_kernel<true> : col_partial_kernel<false>, grid, 256, 0, s, (const void *)in, (void *)dst, rows, p.groups, p.W, p.R);
 }
 
 int launch_col_sum(vrhi_stream_t *st, const ArgView *args, int n_args, const void *params, size_t params_size) {
@@ -801,7 +800,7 @@ int launch_col_sum(vrhi_stream_t *st, const ArgView *args, int n_args, const voi
     VRHI_TRY(stream_arena(st, p.gy * q.cols * 4, nullptr, &payload));
     dst = (float *)payload;
   }
-  VRHI_CUDA(launch_col_partial(st->s, p, (const float *)args[0].ptr, dst, q.rows));
+  VRHI_CUDA(launch_col_partial(chains(st), st->s, p, (const float *)args[0].ptr, dst, q.rows));
   VRHI_TRY(post_launch(st, "col_sum"));
   if (p.gy == 1) return VRHI_OK;
   FinishJobs jobs{};
@@ -888,7 +887,7 @@ extern "C" int vrhi_col_sum_static_scratch(const float *in_device, float *out_de
   // array has to be cleared and whatever an earlier call left behind is never read.
   // (float4 stores: an output that is only 4-byte aligned goes through the array even where one partial row is enough.)
   const bool direct = p.gy == 1 && (!p.vec || reinterpret_cast<uintptr_t>(out_device) % 16 == 0);
-  cudaError_t e = launch_col_partial(s, p, in_device, direct ? out_device : partials, rows);
+  cudaError_t e = launch_col_partial(false, s, p, in_device, direct ? out_device : partials, rows);
   if (e != cudaSuccess) return fail(VRHI_ERR_CUDA, "launch of col_sum_static_scratch (partials) failed: %s", cudaGetErrorString(e));
   if (!direct) {
     FinishJobs jobs{};

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256, 4) vertex_transform_kernel(const float *_
                                                                uint64_t n) {
   __shared__ __align__(16) float tile[3 * kVerts];
   __shared__ Mat4 sm[3];
+  pdl_begin();
   const uint32_t t = threadIdx.x;
   if (t < 48) {
     const float *src = t < 16 ? model : (t < 32 ? view : proj);
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(256, 4) vertex_transform_kernel(const float *_
 }
 
 __global__ void __launch_bounds__(256) flat_color_kernel(const float *__restrict__ color, float4 *__restrict__ out, uint64_t n) {
+  pdl_begin();
   const float4 c = make_float4(color[0], color[1], color[2], 1.0f);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) __stcs(out + k, c);
@@ -107,8 +109,8 @@ int launch_vertex_transform(vrhi_stream_t *st, const ArgView *args, int n_args, 
   for (int k = 0; k < 6; ++k)
     if (args[k].bytes < need[k]) return fail(VRHI_ERR_SIZE, "vertex_transform: argument %d holds %llu bytes, %llu needed", k, (unsigned long long)args[k].bytes, (unsigned long long)need[k]);
   if (!writable(args[4]) || !writable(args[5])) return fail(VRHI_ERR_INVALID, "vertex_transform: an output buffer is read-only");
-  vertex_transform_kernel<<<grid_for(st, (q.n + 3) / 4), 256, 0, st->s>>>((const float *)args[0].ptr, (const float *)args[1].ptr, (const float *)args[2].ptr,
-                                                                (const float *)args[3].ptr, (float4 *)args[4].ptr, (float *)args[5].ptr, q.n);
+  VRHI_CUDA(launch_chained(chains(st), vertex_transform_kernel, dim3(grid_for(st, (q.n + 3) / 4)), 256, 0, st->s, (const float *)args[0].ptr, (const float *)args[1].ptr, (const float *)args[2].ptr,
+                                                                (const float *)args[3].ptr, (float4 *)args[4].ptr, (float *)args[5].ptr, q.n));
   return post_launch(st, "vertex_transform");
 }
 
@@ -120,7 +122,7 @@ int launch_flat_color(vrhi_stream_t *st, const ArgView *args, int n_args, const 
   if (args[0].bytes < 12) return fail(VRHI_ERR_SIZE, "flat_color: the colour needs 12 bytes");
   if (args[1].bytes < q.n * 16) return fail(VRHI_ERR_SIZE, "flat_color: the fragment buffer holds %llu bytes, %llu needed", (unsigned long long)args[1].bytes, (unsigned long long)q.n * 16);
   if (!writable(args[1])) return fail(VRHI_ERR_INVALID, "flat_color: the fragment buffer is read-only");
-  flat_color_kernel<<<grid_for(st, q.n), 256, 0, st->s>>>((const float *)args[0].ptr, (float4 *)args[1].ptr, q.n);
+  VRHI_CUDA(launch_chained(chains(st), flat_color_kernel, dim3(grid_for(st, q.n)), 256, 0, st->s, (const float *)args[0].ptr, (float4 *)args[1].ptr, q.n));
   return post_launch(st, "flat_color");
 }
 

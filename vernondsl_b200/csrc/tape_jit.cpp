@@ -54,8 +54,7 @@ struct Nvrtc {
 struct Driver {
   CUresult (*module_load_data)(CUmodule *, const void *) = nullptr;
   CUresult (*module_get_function)(CUfunction *, CUmodule, const char *) = nullptr;
-  CUresult (*launch_kernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream, void **,
-                            void **) = nullptr;
+  CUresult (*launch_kernel)(const CUlaunchConfig *, CUfunction, void **, void **) = nullptr;
   CUresult (*get_error_string)(CUresult, const char **) = nullptr;
   CUresult (*occupancy)(int *, CUfunction, int, size_t) = nullptr;
   bool ok = false;
@@ -124,7 +123,7 @@ void load_once() {
   if (!g_nvrtc.ok && fallback.ok) g_nvrtc = fallback;
   Driver &d = g_driver;
   d.ok = drv("cuModuleLoadData", &d.module_load_data) && drv("cuModuleGetFunction", &d.module_get_function) &&
-         drv("cuLaunchKernel", &d.launch_kernel) && drv("cuGetErrorString", &d.get_error_string) &&
+         drv("cuLaunchKernelEx", &d.launch_kernel) && drv("cuGetErrorString", &d.get_error_string) &&
          drv("cuOccupancyMaxActiveBlocksPerMultiprocessor", &d.occupancy);
 }
 
@@ -222,7 +221,7 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
   for (unsigned k = 0; k < NI; ++k) s += "const float *__restrict__ in" + str(k) + ", ";
   for (unsigned k = 0; k < NO; ++k) s += "float *__restrict__ out" + str(k) + ", ";
   s += "const " + ULL + " rows, const " + ULL + " groups, const unsigned int W, const unsigned int R, const unsigned int tail, const " + ULL + " cols, const " + ULL + " rem, const unsigned int fold) {\n";
-  if (any_colsum || any_total) s += "  asm volatile(\"griddepcontrol.launch_dependents;\");  // the kernel that adds the partial sums may be launched\n";
+  s += "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");  // a programmatic dependent of the kernel before it, and the next one of it\n  asm volatile(\"griddepcontrol.launch_dependents;\");\n";
   if (form == FLAT) {
     s += "  " + ULL + " i = (" + ULL + ")blockIdx.x * 256u + threadIdx.x;\n  const " + ULL + " step = (" + ULL + ")gridDim.x * 256u;\n";
   } else {
@@ -520,7 +519,16 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   }
   for (uint32_t k = 0; k < q.n_outputs; ++k) args[n_args++] = &out_copy[k];
   args[n_args++] = &rows; args[n_args++] = &groups; args[n_args++] = &W; args[n_args++] = &R; args[n_args++] = &tail; args[n_args++] = &cols; args[n_args++] = &rem; args[n_args++] = &fold;
-  CUresult cr = g_driver.launch_kernel(it->second.fn, (unsigned)gx, (unsigned)gy, 1, 256, 1, 1, 0, reinterpret_cast<CUstream>(st->s), args, nullptr);
+  CUlaunchAttribute attr{};
+  attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig cfg{};
+  cfg.gridDimX = (unsigned)gx; cfg.gridDimY = (unsigned)gy; cfg.gridDimZ = 1;
+  cfg.blockDimX = 256; cfg.blockDimY = 1; cfg.blockDimZ = 1;
+  cfg.hStream = reinterpret_cast<CUstream>(st->s);
+  cfg.attrs = &attr;
+  cfg.numAttrs = chains(st) ? 1 : 0;
+  CUresult cr = g_driver.launch_kernel(&cfg, it->second.fn, args, nullptr);
   if (cr != CUDA_SUCCESS) {
     const char *msg = "?";
     g_driver.get_error_string(cr, &msg);

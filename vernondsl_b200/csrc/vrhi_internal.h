@@ -215,13 +215,15 @@ inline int element_count(uint64_t rows, uint64_t cols, const char *name, uint64_
   return VRHI_OK;
 }
 
-// Programmatic dependent launch of a kernel that finishes what the kernel before it on the stream began
-// (adds up its partial sums).  The blocks of `kern` become resident as soon as every block of the kernel before it
-// has executed pdl_release() or ended, so its launch latency runs under that kernel; it must execute
-// pdl_wait() before it reads anything, which returns when the kernel before it has completed.  Whatever is
-// launched next in the ordinary way finds both finished.
+// Programmatic dependent launch: the blocks of `kern` become resident as soon as every block of the kernel before it on
+// the stream has executed pdl_release() or ended, so its launch latency, about a microsecond, runs under that kernel.  Every
+// thread of a kernel launched so executes pdl_begin() before it touches memory: it waits until the kernel before has
+// completed and its results are visible, and then lets the next one come.  Waiting comes first so that a launch that has
+// begun has everything before it behind it.  Whatever is launched next in the ordinary way finds both finished.
+// Measured on B200 against ordinary launches, calls back to back: tape of [1081,1919] 8.2 -> 6.3 us, vertex stage of 1000003
+// vertices 10.2 -> 8.4, row sums + row maxima + column sums of [1000,1001] 15.4 -> 13.8, 1080p Mandelbrot frame 50.5 -> 48.4.
 template <class Kern, class... Args>
-cudaError_t launch_dependent(Kern kern, dim3 grid, unsigned block, size_t dyn, cudaStream_t s, Args... args) {
+cudaError_t launch_chained(bool chain, Kern kern, dim3 grid, unsigned block, size_t dyn, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
@@ -231,12 +233,21 @@ cudaError_t launch_dependent(Kern kern, dim3 grid, unsigned block, size_t dyn, c
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chain ? 1u : 0u;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
+template <class Kern, class... Args>
+cudaError_t launch_dependent(Kern kern, dim3 grid, unsigned block, size_t dyn, cudaStream_t s, Args... args) {
+  return launch_chained(true, kern, grid, block, dyn, s, args...);
+}
+// An operator's first kernel is chained to whatever came before it, but not in a recording: there the launches of the
+// other streams run beside it, and blocks that only wait would take their places (64 frames of 640 x 320 recorded on
+// two streams: 172 us, and 200 us chained).
+inline bool chains(const vrhi_stream_t *st) { return !st->recording; }
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() { pdl_wait(); pdl_release(); }
 #endif
 
 inline int post_launch(vrhi_stream_t *st, const char *what, int kernels = 1) {
