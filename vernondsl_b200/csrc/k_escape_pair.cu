@@ -21,6 +21,12 @@
 //    INTAKE: 64 fresh pixels of a stolen tile run K checked steps in lock step (most pixels of the
 //    far exterior end there and are stored coalesced); survivors are pushed to the ring with their
 //    state.  Long-lived pixels therefore share warps with other long-lived pixels.
+//  * CYCLES.  Most pixels that reach max_iter do so because their orbit converges, and a converging orbit in binary32
+//    repeats a state bit for bit before long.  The update depends on the state alone, so a valid block that ends on
+//    exactly the state it began with would be repeated for ever: none of its states has escaped, and the count is
+//    max_iter without running the rest.  U = 12 finds cycles of 1, 2, 3, 4, 6 and 12 steps, those of the set's
+//    largest components.  Same counts; measured on B200, whole-set views against running every step: 1080p, 256 steps
+//    48.4 -> 40.0 us, 1024 steps 144 -> 83 us; 4096 x 4096, 1024 steps 851 -> 415 us.
 //  * WORK STEALING.  Warps pull batches of up to 24 tiles (1536 pixels of one row) from a global
 //    counter.  Nothing here waits on another warp or block: no spin loops, no barriers.
 //
@@ -52,6 +58,9 @@ constexpr int kPairPool = 128;  // pool entries per warp: a refill wants up to 6
 template <int KIND, int OUT, int U, int T, int K, int MODE, bool WIRE, int EX, int NBLK>
 __global__ void __launch_bounds__(256, 4) escape_pair_kernel(EscapeDev p, void *image, uint32_t *work_counter, uint16_t *wire) {
   constexpr bool PER_PIXEL_C = (KIND == VRHI_ESCAPE_MANDELBROT);
+  // Julia images have converging orbits only where c lies in the Mandelbrot set; the comparison costs the others 3 to 5 %
+  // (1080p, 256 steps: 35.8 -> 37.0 us; 4096 x 4096: 163.8 -> 170.1)
+  constexpr bool CYCLES = KIND == VRHI_ESCAPE_MANDELBROT;
   begin_launch(p);
   __shared__ float4 s_pool[8][kPairPool];  // zr, zi, pixel index, count: one 16-byte access per entry
   __shared__ float2 s_c[PER_PIXEL_C ? 8 : 1][PER_PIXEL_C ? kPairPool : 1];
@@ -250,6 +259,13 @@ __global__ void __launch_bounds__(256, 4) escape_pair_kernel(EscapeDev p, void *
         run1 = run1 && (s1 <= bound) && (cnt1 <= fast_limit);
         cnt0 += run0 ? (uint32_t)U : 0u;
         cnt1 += run1 ? (uint32_t)U : 0u;
+        if (CYCLES) {
+          // a block that ends on the state it began with: see CYCLES at the top
+          const f32x2 d = (ZR ^ CKR) | (ZI ^ CKI);
+          const bool cycle0 = run0 && (uint32_t)d == 0u, cycle1 = run1 && (uint32_t)(d >> 32) == 0u;
+          if (cycle0) { cnt0 = max_iter; run0 = false; }
+          if (cycle1) { cnt1 = max_iter; run1 = false; }
+        }
         ZR = select2(run0, run1, ZR, CKR);
         ZI = select2(run0, run1, ZI, CKI);
         if (nb + 1 < NBLK) pair_squares<MODE>(ZR, ZI, NZ, A, B);
