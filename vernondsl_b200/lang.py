@@ -285,9 +285,12 @@ def min(a, b):  # noqa: A001
 
 # --- analysis helpers ---------------------------------------------------------------------------
 
+_ZERO, _ONE = Fraction(0), Fraction(1)
+
+
 def _affine(e, n_index: int) -> Optional[List[Fraction]]:
     """[c0, c_index0, c_index1, ...] if e is affine in the loop indices with numeric coefficients."""
-    zero = [Fraction(0)] * (n_index + 1)
+    zero = [_ZERO] * (n_index + 1)
     if _is_num(e):
         return [Fraction(float(e)) if not isinstance(e, (int, Fraction)) else Fraction(e)] + zero[1:]
     if not isinstance(e, Sym):
@@ -296,7 +299,7 @@ def _affine(e, n_index: int) -> Optional[List[Fraction]]:
         return _affine(e.value, n_index)
     if e.op == "index":
         out = list(zero)
-        out[1 + e.value] = Fraction(1)
+        out[1 + e.value] = _ONE
         return out
     if e.op in ("add", "sub"):
         a, b = _affine(e.args[0], n_index), _affine(e.args[1], n_index)
@@ -333,9 +336,9 @@ def _poly(e, names) -> Optional[Dict[Tuple[int, int], Fraction]]:
     if e.op == "const":
         return _poly(e.value, names)
     if e.op == "zvar":
-        return {(1, 0): Fraction(1)} if e.value == 0 else {(0, 1): Fraction(1)}
+        return {(1, 0): _ONE} if e.value == 0 else {(0, 1): _ONE}
     if e.op == "cconst":  # component of the constant c: a fresh symbol, carried as a tagged monomial
-        return {("c", e.value): Fraction(1)}
+        return {("c", e.value): _ONE}
     if e.op == "neg":
         a = _poly(e.args[0], names)
         return None if a is None else {k: -v for k, v in a.items()}
@@ -345,7 +348,7 @@ def _poly(e, names) -> Optional[Dict[Tuple[int, int], Fraction]]:
             return None
         out = dict(a)
         for k, v in b.items():
-            out[k] = out.get(k, Fraction(0)) + (v if e.op == "add" else -v)
+            out[k] = out.get(k, _ZERO) + (v if e.op == "add" else -v)
         return {k: v for k, v in out.items() if v != 0}
     if e.op == "mul":
         a, b = _poly(e.args[0], names), _poly(e.args[1], names)
@@ -363,7 +366,7 @@ def _poly(e, names) -> Optional[Dict[Tuple[int, int], Fraction]]:
                         return None  # c times a variable: not the quadratic map
                 else:
                     k = (ka[0] + kb[0], ka[1] + kb[1])
-                out[k] = out.get(k, Fraction(0)) + va * vb
+                out[k] = out.get(k, _ZERO) + va * vb
         return {k: v for k, v in out.items() if v != 0}
     return None
 
@@ -389,7 +392,7 @@ class _Reads:
         """Only values that say all there is to know by being the same object, or an equal number."""
         if isinstance(v, Field):
             self.fields[id(v)] = (v, v.shape, v.dtype)
-        elif not (_is_num(v) or isinstance(v, (_Func, types.ModuleType)) or any(v is f for f in _known())):
+        elif not (_is_num(v) or isinstance(v, (_Func, types.ModuleType)) or id(v) in _KNOWN):
             raise _Depends()
         return v
 
@@ -429,9 +432,8 @@ class _Reads:
         return True
 
 
-def _known():
-    """The functions of this module a kernel may call."""
-    return (Vector, cos, sin, sqrt, exp, log, tanh)
+# the functions of this module that a kernel with a kept plan may call (they live as long as the module)
+_KNOWN = {id(f): f for f in (Vector, cos, sin, sqrt, exp, log, tanh)}
 
 
 class _Walker:
@@ -443,7 +445,7 @@ class _Walker:
         self.closure = dict(zip(fn.__code__.co_freevars, fn.__closure__)) if fn.__closure__ else {}
         # every enclosing name is part of the environment, as a kernel body may not rebind one it has not bound before
         self.env: Dict[str, Any] = {} if reads else {name: cell.cell_contents for name, cell in self.closure.items()}
-        values = _bind(fn, fdef, call_args)
+        values = _bind(fn, _floats(fdef), call_args)
         for k, (a, value) in enumerate(zip(fdef.args.args, values)):
             if reads:
                 if not _is_num(value):
@@ -517,7 +519,7 @@ class _Walker:
             args = [self.ev(a) for a in node.args]
             if isinstance(f, _Func):
                 return f.inline(args, self.reads)
-            if self.reads and not any(f is g for g in _known()):
+            if self.reads and id(f) not in _KNOWN:
                 raise _Depends()
             return f(*args)
         raise LangError(f"unsupported expression: {ast.dump(node)[:80]}")
@@ -563,27 +565,30 @@ def func(fn):
     return _Func(fn)
 
 
-def _bind(fn, fdef, call_args) -> list:
+def _floats(fdef) -> List[bool]:
+    """Which parameters are annotated as float."""
+    return [isinstance(a.annotation, ast.Name) and a.annotation.id == "float" for a in fdef.args.args]
+
+
+def _bind(fn, floats: List[bool], call_args) -> list:
     """The kernel's arguments as its body sees them: floats in binary32."""
-    params = fdef.args.args
-    if len(params) != len(call_args):
-        raise TypeError(f"{fn.__name__}() takes {len(params)} arguments, {len(call_args)} given")
-    return [f32(v) if (isinstance(a.annotation, ast.Name) and a.annotation.id == "float") or isinstance(v, float) else v
-            for a, v in zip(params, call_args)]
+    if len(floats) != len(call_args):
+        raise TypeError(f"{fn.__name__}() takes {len(floats)} arguments, {len(call_args)} given")
+    return [f32(v) if is_float or isinstance(v, float) else v for is_float, v in zip(floats, call_args)]
 
 
 class _Plan:
     """An escape-time launch as a walk with ``_Uniform`` arguments found it: the parameter block, how the constant's two
     components follow from the arguments, and what the walk read from outside the kernel."""
 
-    def __init__(self, reads: _Reads, field: Field, params, constant, text: str):
-        self.reads, self.field, self.params, self.constant, self.text = reads, field, params, constant, text
+    def __init__(self, reads: _Reads, field: Field, params, constant, text: str, floats: List[bool]):
+        self.reads, self.field, self.params, self.constant, self.text, self.floats = reads, field, params, constant, text, floats
 
-    def instance(self, fn, fdef, call_args):
+    def instance(self, fn, call_args):
         """The parameter block for other arguments, or None where the walk has to be repeated."""
         if not self.reads.unchanged():
             return None
-        values = _bind(fn, fdef, call_args)
+        values = _bind(fn, self.floats, call_args)
         if not all(type(v) in (f32, int, float) for v in values):
             return None
         c = [x if of is None else float(f32(float(of(values)))) for x, of in zip((self.params.cr, self.params.ci), self.constant)]
@@ -605,30 +610,29 @@ class Kernel:
         self.last_plan: Optional[str] = None
         self.last_params = None
         self.last_tape = None
-        self._fdef: Optional[ast.FunctionDef] = None
+        self._fdef: Optional[ast.FunctionDef] = None     # the parsed source, kept where there is no plan
         self._plan: Optional[_Plan] = None
         self._plannable = True      # False once a walk succeeded that cannot be kept: the next calls do not try again
 
     def __call__(self, *args):
         st = None if _state["plan_only"] else _runtime()[1]     # None: lower only
-        if self._fdef is None:
-            self._fdef = _parse(self.fn)
         plan = self._plan
         if plan is not None:
-            p = plan.instance(self.fn, self._fdef, args)
+            p = plan.instance(self.fn, args)
             if p is not None:
                 self.last_plan, self.last_params = plan.text, p
                 self._launch_escape(st, plan.field, p)
                 return
         self._plan = None
+        fdef = self._fdef if self._fdef is not None else _parse(self.fn)
         if self._plannable:
             try:
-                self._walk(_Walker(self.fn, self._fdef, args, _Reads()), st)
+                self._walk(_Walker(self.fn, fdef, args, _Reads()), st)
                 return
             except (_Depends, LangError):
                 pass        # walked again with the arguments' values, which also says what is wrong where something is
-        self._walk(_Walker(self.fn, self._fdef, args), st)
-        self._plannable = False
+        self._walk(_Walker(self.fn, fdef, args), st)
+        self._plannable, self._fdef = False, fdef
 
     def _walk(self, w: _Walker, st):
         body = [s for s in w.fdef.body if not (isinstance(s, ast.Expr) and isinstance(s.value, ast.Constant))]
@@ -784,7 +788,7 @@ class Kernel:
         self.last_plan = f"escape_time kind={'julia' if kind == L.JULIA else 'mandelbrot'} {cols}x{rows} transposed={transposed}"
         self.last_params = p
         if w.reads:
-            self._plan = _Plan(w.reads, fld, p, constant, self.last_plan)
+            self._plan = _Plan(w.reads, fld, p, constant, self.last_plan, _floats(w.fdef))
         self._launch_escape(st, fld, p)
 
     # -- elementwise shape -----------------------------------------------------------------------
