@@ -73,7 +73,9 @@ namespace vrhi {
 constexpr size_t kCtrlBytes = 256;
 // control-word indices (uint32) inside the arena's control block
 enum { CTRL_STATUS = 0, CTRL_WORK0 = 1, CTRL_WORK1 = 2, CTRL_DONE = 3, CTRL_WAIT_OK = 4,
-       CTRL_ESCAPE_RING = 8 /* 8 work counters, one per launch of a run of overlapping escape-time launches */ };
+       CTRL_ESCAPE_RING = 8 /* 8 work counters, one per launch of a run of overlapping escape-time launches */,
+       CTRL_COL_TICKETS = 24 /* kColTickets counters of finished blocks, one per tile of a column sum; 0 between launches */ };
+constexpr unsigned kColTickets = 40;
 
 int fail(int code, const char *fmt, ...) __attribute__((format(printf, 2, 3)));
 void clear_error();
