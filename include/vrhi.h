@@ -242,8 +242,8 @@ typedef struct vrhi_escape_params {
   uint32_t chunk_rows, chunk_first, chunk_step, chunk_count;
   uint32_t flags; /* VRHI_ESCAPE_FLAG_* */
 } vrhi_escape_params;
-/* Run the kernel that tests on every step even where the faster regrouping kernel applies
- * (exact mode, NORM2_GT with bound >= 4, |c| <= 1.5).  Results are identical either way. */
+/* Run the kernel that tests on every step even where a faster one applies (a limit of 4 or more on
+ * a+b, a constant for which escape is final).  Results are identical either way. */
 #define VRHI_ESCAPE_FLAG_CHECKED_ONLY 1u
 /* The real axis runs along the rows and the imaginary axis along the columns: pixel (row j,
  * column i) has real part y0 + j*dy and imaginary part x0 + i*dx.  This is the memory order of a

@@ -13,7 +13,7 @@
 //
 // This file holds the operator's launcher and the fully checked kernel: one pixel per lane, a test
 // on every step.  That kernel accepts every parameter combination and is the path of record for
-// parameters the regrouping kernel (k_escape_pair.cu) cannot take.
+// parameters the kernels with unchecked blocks (k_escape_pair.cu, k_escape_block.cu) cannot take.
 #include <cfloat>
 #include <cmath>
 #include <cstdlib>
@@ -162,9 +162,9 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
   // and pool and then loses nothing to pixels that outlive their neighbours; the block kernel (k_escape_block.cu) runs a
   // warp as long as its slowest pixel.  So regroup where pixels may run long and every warp sees many tiles.  Measured on B200,
   // regrouping against blocks, Julia / Mandelbrot in us:
-  //   640 x 320     256 steps: 13.3 vs 10.9 / 13.4 vs 9.5       1024: 30.4 vs 31.3 / 42.8 vs 30.4
-  //   1920 x 1080   128: 31.1 vs 27.4 / 34.6 vs 30.4            256: 36.5 vs 43.3 / 48.9 vs 47.4     1024: 55 vs 103 / 143 vs 151
-  //   4096 x 4096   64: 107 vs 106 / 141 vs 127                 128: 130 vs 154 / 183 vs 188         256: 164 vs 251 / 283 vs 303
+  //   640 x 320     256 steps: 13.1 vs 10.9 / 15.2 vs 9.5       1024: 29.8 vs 31.3 / 49.6 vs 30.4
+  //   1920 x 1080   128: 31.1 vs 27.4 / 32.2 vs 30.4            256: 36.5 vs 43.3 / 39.9 vs 47.4     1024: 55 vs 103 / 83 vs 151
+  //   4096 x 4096   64: 107 vs 106 / 141 vs 127                 128: 130 vs 154 / 167 vs 188         256: 164 vs 251 / 212 vs 303
   const uint64_t pixels = (uint64_t)q.width * p.rows_owned;
   //   128 x 64      256: 7.2 vs 6.8 / 7.4 vs 7.0                1024: 14.9 vs 19.4 / 18.3 vs 23.6 (one tile per warp: the
   //                 length of a warp's chain of blocks and votes is all there is)

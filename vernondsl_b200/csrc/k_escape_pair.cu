@@ -1,8 +1,9 @@
 // Escape-time map, regrouping kernel: two pixels per lane in packed binary32 pairs (sm_100a).
 //
 // Loop rules as in k_escape.cu (fractal.py:11-25): test before update, count the updates, square
-// as (z0*z0 - z1*z1, (z1*z0)*2).  Accepted parameters: test "a+b > bound" with bound >= 4,
-// |c| <= 1.5 (Mandelbrot pixels with a larger constant are finished at intake), max_iter >= 64.
+// as (z0*z0 - z1*z1, (z1*z0)*2).  Accepted parameters: a limit of 4 or more on a+b, max_iter >= 12, a
+// Julia constant for which escape is final (EscapeDev::c2_unsafe_lo; Mandelbrot pixels whose constant is not are
+// finished at intake).
 //
 // Iteration counts inside a warp differ by orders of magnitude near the set, so one pixel per lane
 // with a test on every step leaves most lanes idle (about 36 % lane efficiency on the 16384^2
@@ -10,9 +11,9 @@
 //
 //  * UNCHECKED BLOCKS.  A slot runs U updates with no test and no counter (six arithmetic
 //    operations per update).  One test at the end decides whether the whole block was valid.  That
-//    is exact because, for bound >= 4 and |c| <= 1.5, escape is monotonic even in binary32: once
-//    a+b > bound then |z'| >= |z|^2 - |c| > 1.2|z|, so every later a+b is larger still, or Inf/NaN,
-//    and the test is written !(s <= bound) so that NaN counts as escaped.  A slot whose block failed
+//    is exact because, for limits of 4 and more and all but a thin ring of constants, escape is final even in
+//    binary32 (EscapeDev::c2_unsafe_lo): every later a+b is larger still, or Inf/NaN, and the test is
+//    written !(s <= limit) so that NaN counts as escaped.  A slot whose block failed
 //    the test (or would pass max_iter) is put back on its checkpoint and marked "finishing".
 //  * CHECKED BLOCKS.  When at least T slots are finishing or empty, the warp runs one block of U
 //    steps with the test and the counter on every step; slots still in flight simply advance,
