@@ -1,7 +1,7 @@
 // Row reductions, softmax and column sums of a row-major [rows][cols] float matrix, sm_100a.
 //
 // HBM-bound: every kernel reads a row from HBM once, holds what it needs of it in registers and keeps many 16-byte loads in
-// flight.  Rows whose length is no multiple of 8 start anywhere in a 32-byte sector; their kernels (EDGE) split a row into
+// flight.  Rows whose length is no multiple of 4 start at any 4-byte boundary; their kernels (EDGE) split a row into
 // up to three elements in front of the first 16-byte boundary, float4 groups, and up to three elements behind them, so
 // every length runs at the speed of the round ones.  By row length:
 //   up to 64               a few lanes per row, single elements (row_narrow_kernel)
@@ -571,8 +571,10 @@ static int launch_rows(vrhi_stream_t *st, const float *in, float *osum, float *o
   if (cols <= 16) VRHI_CUDA(launch_chained(chains(st), row_narrow_kernel<4, 4, WHAT>, dim3(row_grid(rows, 64)), 256, 0, st->s, in, osum, omax, osoft, rows, (uint32_t)cols));
   else if (cols <= 64) VRHI_CUDA(launch_chained(chains(st), row_narrow_kernel<8, 8, WHAT>, dim3(row_grid(rows, 32)), 256, 0, st->s, in, osum, omax, osoft, rows, (uint32_t)cols));
   else if constexpr ((WHAT & ROW_SOFTMAX) != 0) {
-    VRHI_CUDA((cols % 8 != 0 ? launch_softmax<WHAT, true>(st, in, osum, omax, osoft, rows, cols)  // rows that start inside a 32-byte sector
-                             : launch_softmax<WHAT, false>(st, in, osum, omax, osoft, rows, cols)));
+    // EDGE: rows that start off a 16-byte boundary, and long ones that start inside a 32-byte sector.  Short rows of 4, 12, 20,
+    // ... elements lose more to its bookkeeping than half sectors cost ([133152,252] 42 us without, 54 with).
+    const bool edge = cols % 4 != 0 || (cols % 8 != 0 && cols > 8192);
+    VRHI_CUDA((edge ? launch_softmax<WHAT, true>(st, in, osum, omax, osoft, rows, cols) : launch_softmax<WHAT, false>(st, in, osum, omax, osoft, rows, cols)));
   } else {
     constexpr bool MAX = WHAT == ROW_MAX;
     float *out = MAX ? omax : osum;
