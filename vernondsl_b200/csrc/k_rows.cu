@@ -220,7 +220,7 @@ struct RowExp {
 // shared arrays (sum, max, normaliser), one CTA barrier each; partials are combined in a fixed
 // order, so results do not depend on scheduling.
 template <int NV, int WPR, int WHAT, bool EDGE>
-__global__ void __launch_bounds__(WPR > 8 ? 32 * WPR : 256, WPR > 8 ? 3 : WPR > 4 ? 5 : 4) row_group_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
+__global__ void __launch_bounds__(WPR > 8 ? 32 * WPR : 256, WPR > 8 ? 3 : WPR > 4 && NV <= 5 ? 5 : 4) row_group_kernel(const float *__restrict__ in, float *__restrict__ out_sum,
                                                                            float *__restrict__ out_max, float *__restrict__ out_soft,
                                                                            uint64_t rows, uint32_t cols) {
   constexpr int GROUPS = WPR > 8 ? 1 : 8 / WPR;
@@ -537,7 +537,8 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
   // Registers for a row of the block's: 64 per thread with 8 float4 (four blocks of 256 threads per SM), 40 with 5 (three of 512,
   // six of 256).  One more block per SM in another phase is worth more than any other choice here: [4096,10000] 50.7 us
   // with three blocks of 512 threads per SM, 60 us with two.
-  const uint32_t wpr = most4 <= 256 ? 1 : most4 <= 512 ? 2 : most4 <= 1024 ? 4 : most4 <= 1280 ? 8 : 16;
+  // (8 warps with 8 float4, whole groups only: [4790,7004] 49.5 us, 16 warps with 4 float4 53)
+  const uint32_t wpr = most4 <= 256 ? 1 : most4 <= 512 ? 2 : most4 <= 1024 ? 4 : most4 <= (EDGE ? 1280 : 1792) ? 8 : 16;
   const uint32_t nv = (uint32_t)((most4 + 32u * wpr - 1) / (32u * wpr));
   // one CTA per group of rows, not a persistent grid: measured on B200, letting the hardware
   // scheduler stream CTAs (each loads, reduces, writes and leaves) beats a resident grid whose
@@ -547,7 +548,7 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
 #define GROUP_NV(WPR)                     \
   do {                                    \
     if (nv <= 5) GROUP_LAUNCH(5, WPR);    \
-    else if (nv <= 6) GROUP_LAUNCH(6, WPR); \
+    else if (EDGE && nv <= 6) GROUP_LAUNCH(6, WPR); /* whole groups with 6: [22369,1500] 57 us, with 8 43 */ \
     else GROUP_LAUNCH(8, WPR);            \
   } while (0)
   if (wpr == 1) {
@@ -557,7 +558,8 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
     else GROUP_LAUNCH(8, 1);
   } else if (wpr == 2) GROUP_NV(2);
   else if (wpr == 4) GROUP_NV(4);
-  else if (wpr == 8) GROUP_LAUNCH(5, 8);
+  else if (wpr == 8 && (EDGE || nv <= 5)) GROUP_LAUNCH(5, 8);
+  else if (wpr == 8) GROUP_LAUNCH(8, 8);
   else if (nv <= 3) GROUP_LAUNCH(3, 16);
   else if (nv <= 4) GROUP_LAUNCH(4, 16);
   else GROUP_LAUNCH(5, 16);
