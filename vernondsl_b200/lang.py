@@ -218,8 +218,12 @@ class _Uniform:
     __eq__ = __ne__ = __lt__ = __le__ = __gt__ = __ge__ = __getattr__ = _depends
 
 
+_NUMBERS = frozenset((int, float, bool, f32, Fraction))
+
+
 def _is_num(v) -> bool:
-    return isinstance(v, (int, float, np.floating, np.integer, Fraction))
+    # the usual types first: isinstance takes a third of a microsecond to say that something is no Fraction (an abstract base class)
+    return type(v) in _NUMBERS or (type(v) is not Sym and isinstance(v, (int, float, np.floating, np.integer, Fraction)))
 
 
 class Vector:
@@ -374,8 +378,31 @@ def _poly(e, names) -> Optional[Dict[Tuple[int, int], Fraction]]:
 # ------------------------------------------------------------------------------------------------
 # The walker: a small evaluator over the subset of Python that kernel bodies use.
 
+def _block(lines: List[str]) -> str:
+    """The function that begins on the first line (its decorators included): everything up to the first line of code behind
+    its ``def`` that is indented no deeper.  ``inspect.getblock`` finds the same end by tokenizing, which takes longer than
+    parsing the block does.  A line inside a string, inside brackets or behind a backslash may stop the search too early;
+    what it then returns is no complete statement."""
+    margin = len(lines[0]) - len(lines[0].lstrip(" "))
+    header, end = True, 0
+    for k, line in enumerate(lines):
+        text = line.lstrip(" ")
+        if not text.strip() or text[0] == "#":
+            continue
+        if len(line) - len(text) <= margin:
+            if not header:
+                break
+            header = not text.startswith(("def ", "async "))
+        end = k + 1
+    return "".join(lines[:end])
+
+
 def _parse(fn) -> ast.FunctionDef:
-    tree = ast.parse(textwrap.dedent(inspect.getsource(fn)))
+    try:
+        lines, first = inspect.findsource(inspect.unwrap(fn))
+        tree = ast.parse(textwrap.dedent(_block(lines[first:])))
+    except SyntaxError:
+        tree = ast.parse(textwrap.dedent(inspect.getsource(fn)))
     return next(n for n in tree.body if isinstance(n, ast.FunctionDef))
 
 
