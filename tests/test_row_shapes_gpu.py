@@ -89,3 +89,35 @@ def test_infinities_nan_and_the_lowest_value(dev, stream, cols):
     assert abs(float(p[6].astype(np.float64).sum()) - 1) < 1e-5
     for b in (X, S, M, P):
         b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cols", [67, 1001, 10007, 20483, 32741, 40001, 50002, 140003])
+@pytest.mark.parametrize("special", [np.nan, np.inf, -np.inf])
+def test_special_values_at_the_ends_of_rows_of_every_phase(dev, stream, cols, special):
+    """The first and the last element of a row lie in front of and behind its float4 groups, how many of them there are
+    depends on where the row starts: eight rows of one length, four with the value first and four with it last."""
+    f = np.float32
+    x = np.random.default_rng(cols).standard_normal((8, cols)).astype(f)
+    x[:4, 0] = special
+    x[4:, -1] = special
+    rows = x.shape[0]
+    X = dev.from_numpy(x, L.INPUT)
+    S, M, M2 = (dev.empty(rows, f, L.OUTPUT) for _ in range(3))
+    P, Q = (dev.empty((rows, cols), f, L.OUTPUT) for _ in range(2))
+    ops.row_stats_softmax(stream, X, S, M, P, rows, cols)
+    ops.row_max(stream, X, M2, rows, cols)
+    ops.row_softmax(stream, X, Q, rows, cols)
+    stream.check()
+    want = np.fmax.reduce(x, axis=1)
+    assert np.array_equal(M.download(), want) and np.array_equal(M2.download(), want)
+    s, p, q = S.download(), P.download(), Q.download()
+    if special == -np.inf:
+        assert (s == -np.inf).all() and (p[:4, 0] == 0).all() and (p[4:, -1] == 0).all()
+        assert (np.abs(p.astype(np.float64).sum(1) - 1) < 1e-5).all()
+    else:      # x - max is NaN at the value itself, so the row's normaliser is
+        assert (np.isnan(s) if special != special else s == special).all()
+        assert np.isnan(p).all()
+    assert np.array_equal(p, q, equal_nan=True)
+    for b in (X, S, M, M2, P, Q):
+        b.close()

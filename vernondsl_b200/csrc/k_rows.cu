@@ -412,13 +412,14 @@ __global__ void __launch_bounds__(512, 3) row_two_pass_kernel(const float *__res
   for (uint64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const uint64_t first = r * cols;
     const uint32_t head = EDGE ? (4u - (uint32_t)(first & 3u)) & 3u : 0u;
-    const uint64_t n4 = (cols - head) >> 2, edges = head + ((cols - head) & 3u), shift = EDGE ? ((first + head) >> 2) & 7u : 0u;
-    const bool has_edge = t < edges;
+    const uint64_t n4 = (cols - head) >> 2, edges = EDGE ? head + ((cols - head) & 3u) : 0u, shift = EDGE ? ((first + head) >> 2) & 7u : 0u;
+    const bool has_edge = EDGE && t < edges;
     const uint64_t at = first + (t < head ? t : 4u * n4 + t);
     const float4 *src = reinterpret_cast<const float4 *>(in + first + head);
     float e = has_edge ? __ldg(in + at) : 0.f;
-    float s = e, m = has_edge ? e : -INFINITY, z = has_edge ? 1.f : 0.f;
-    if (has_edge && e != e) z = e;  // a NaN is not its own maximum
+    // the edge enters like any other element: a NaN is no maximum, and NaN and +inf make the sum NaN
+    float s = e, m = has_edge ? fmaxf(e, -INFINITY) : -INFINITY;
+    float z = has_edge ? expf(e - (m == -INFINITY ? 0.f : m)) : 0.f;
     for (uint64_t c0 = 0; c0 < n4 + shift; c0 += T * U) {
       float4 v[U];
       float chunk = -INFINITY;
