@@ -121,3 +121,23 @@ def test_special_values_at_the_ends_of_rows_of_every_phase(dev, stream, cols, sp
     assert np.array_equal(p, q, equal_nan=True)
     for b in (X, S, M, M2, P, Q):
         b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cols", [40001, 50002, 140003])
+@pytest.mark.parametrize("at", [0, -1])
+def test_a_nan_hides_no_maximum_of_its_own_thread(dev, stream, cols, at):
+    """Rows long enough for two passes: the thread that holds the element in front of or behind the groups also holds one
+    group of the first few hundred behind the 2016th element; the maximum goes through all of them, for every phase."""
+    f = np.float32
+    x = np.random.default_rng(cols).standard_normal((64, cols)).astype(f)
+    x[:, at] = np.nan
+    x[np.arange(64), 2016 + np.arange(64)] = 9.0
+    X = dev.from_numpy(x, L.INPUT)
+    S, M = dev.empty(64, f, L.OUTPUT), dev.empty(64, f, L.OUTPUT)
+    P = dev.empty((64, cols), f, L.OUTPUT)
+    ops.row_stats_softmax(stream, X, S, M, P, 64, cols)
+    stream.check()
+    assert (M.download() == 9.0).all()
+    for b in (X, S, M, P):
+        b.close()
