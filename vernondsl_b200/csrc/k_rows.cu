@@ -518,8 +518,9 @@ static cudaError_t launch_stream_nv(vrhi_stream_t *st, const float *in, float *o
 
 template <int T, int WHAT, bool EDGE>
 static cudaError_t launch_stream(vrhi_stream_t *st, const float *in, float *osum, float *omax, float *osoft, uint64_t rows, uint32_t cols, uint64_t most4) {
-  const uint64_t nv = (most4 + T - 1) / T;
-  if (nv <= 5) return launch_stream_nv<T, 5, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
+  const uint64_t nv = (most4 + T - 1) / T;  // 512 threads: 2561 groups or more
+  if constexpr (T > 512)
+    if (nv <= 5) return launch_stream_nv<T, 5, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
   if (nv <= 6) return launch_stream_nv<T, 6, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
   if (nv <= 7) return launch_stream_nv<T, 7, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
   return launch_stream_nv<T, 8, WHAT, EDGE>(st, in, osum, omax, osoft, rows, cols);
@@ -549,21 +550,29 @@ static cudaError_t launch_softmax(vrhi_stream_t *st, const float *in, float *osu
 #define GROUP_NV(WPR)                     \
   do {                                    \
     if (nv <= 5) GROUP_LAUNCH(5, WPR);    \
-    else if (EDGE && nv <= 6) GROUP_LAUNCH(6, WPR); /* whole groups with 6: [22369,1500] 57 us, with 8 43 */ \
-    else GROUP_LAUNCH(8, WPR);            \
+    if constexpr (EDGE) { /* whole groups with 6: [22369,1500] 57 us, with 8 43 */ \
+      if (nv <= 6) GROUP_LAUNCH(6, WPR);  \
+    }                                     \
+    GROUP_LAUNCH(8, WPR);                 \
   } while (0)
   if (wpr == 1) {
     if (nv <= 1) GROUP_LAUNCH(1, 1);
-    else if (nv <= 2) GROUP_LAUNCH(2, 1);
-    else if (nv <= 4) GROUP_LAUNCH(4, 1);
-    else GROUP_LAUNCH(8, 1);
-  } else if (wpr == 2) GROUP_NV(2);
-  else if (wpr == 4) GROUP_NV(4);
-  else if (wpr == 8 && (EDGE || nv <= 5)) GROUP_LAUNCH(5, 8);
-  else if (wpr == 8) GROUP_LAUNCH(8, 8);
-  else if (nv <= 3) GROUP_LAUNCH(3, 16);
-  else if (nv <= 4) GROUP_LAUNCH(4, 16);
-  else GROUP_LAUNCH(5, 16);
+    if (nv <= 2) GROUP_LAUNCH(2, 1);
+    if (nv <= 4) GROUP_LAUNCH(4, 1);
+    GROUP_LAUNCH(8, 1);
+  }
+  if (wpr == 2) GROUP_NV(2);
+  if (wpr == 4) GROUP_NV(4);
+  // 8 warps have up to 1280 groups with edges (5 per thread) and up to 1792 without (7), 16 warps what is above
+  if (wpr == 8) {
+    if constexpr (!EDGE)
+      if (nv > 5) GROUP_LAUNCH(8, 8);
+    GROUP_LAUNCH(5, 8);
+  }
+  if constexpr (EDGE)
+    if (nv <= 3) GROUP_LAUNCH(3, 16);
+  if (nv <= 4) GROUP_LAUNCH(4, 16);
+  GROUP_LAUNCH(5, 16);
 #undef GROUP_NV
 #undef GROUP_LAUNCH
 }
