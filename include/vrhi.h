@@ -359,7 +359,9 @@ typedef struct vrhi_tape_params {
 /* A tape normally runs as a kernel compiled for it at first use (NVRTC, cached; values in
  * registers, HBM-bound).  This flag, or VRHI_TAPE_JIT=0 in the environment, selects the
  * interpreting kernel instead, which is also what runs where NVRTC is not installed, for unaligned
- * arrays and for a few hundred elements in rows of no multiple of 4.  Both give the same bits. */
+ * arrays and for a few hundred elements in rows of no multiple of 4, and what is recorded where a tape
+ * that has never run meets a recording.  Both give the same bits.  Constants are arguments of the compiled
+ * kernel: tapes that differ in nothing else share it. */
 #define VRHI_TAPE_FLAG_INTERPRET 1u
 #define VRHI_TAPE_FLAG_TOTALS 2u
 /* Tapes compiled so far in this process, launches of compiled tapes (those over rows of a multiple of 4

@@ -12,6 +12,9 @@
 // the tape says so, and the transcendental primitives are the same functions (tape_math.cuh is
 // compiled into both).  The two paths therefore produce the same bits.
 //
+// The tape's constants are no part of the kernel: they are passed by value at each launch.  Two tapes that differ in nothing
+// else, such as the frames of a loop with a moving uniform, share one kernel.
+//
 // NVRTC and the driver entry points are looked up at run time (dlopen, cudaGetDriverEntryPoint):
 // the library neither links against them nor needs them unless a tape is launched.  Where NVRTC is
 // not installed the interpreter runs instead; VRHI_TAPE_JIT=0 in the environment, or
@@ -129,17 +132,11 @@ void load_once() {
 
 std::string v(unsigned k) { return "v" + std::to_string(k); }
 
-// One SSA instruction as a C expression over the values v<k>.
-std::string expression(const vrhi_tape_instr &I) {
+// One SSA instruction as a C expression over the values v<k>; `constant` is the name of a constant's value.
+std::string expression(const vrhi_tape_instr &I, const std::string &constant) {
   const std::string a = v(I.a), b = v(I.b), c = v(I.c);
   switch (I.op) {
-    case VRHI_T_CONST: {
-      uint32_t bits;
-      memcpy(&bits, &I.imm, 4);
-      char buf[48];
-      snprintf(buf, sizeof buf, "__int_as_float((int)0x%08xu)", bits);
-      return buf;
-    }
+    case VRHI_T_CONST: return constant;
     case VRHI_T_ADD: return "__fadd_rn(" + a + ", " + b + ")";
     case VRHI_T_SUB: return "__fsub_rn(" + a + ", " + b + ")";
     case VRHI_T_MUL: return "__fmul_rn(" + a + ", " + b + ")";
@@ -189,7 +186,8 @@ unsigned super_rows_of(uint64_t cols) { return cols % 4 == 0 ? 1 : cols % 2 == 0
 // loaded once per thread, column vectors once per row.  An output is stored, or (colsum_mask) added up over the rows
 // in a register, over the R rows of the block in shared memory, and written as one partial row per block row, or
 // (total_mask) added up over everything the block visits and written as one partial value per block.
-std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
+// `show_constants`: the values of this tape's constants as comments (they are no part of a compiled text).
+std::string generate(const vrhi_tape_params &q, Form form, int unroll, bool show_constants = false) {
   const unsigned NI = q.n_inputs, NO = q.n_outputs, NT = q.n_instr;
   const unsigned P = super_rows_of(q.cols);
   const std::vector<std::string> comps{".x", ".y", ".z", ".w"};
@@ -210,16 +208,36 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
   bool any_colsum = false, any_total = false;
   for (unsigned k = 0; k < NO; ++k) { any_colsum = any_colsum || colsum(k); any_total = any_total || total(k); }
 
+  unsigned NC = 0;
+  for (unsigned t = 0; t < NT; ++t) NC += q.instr[t].op == VRHI_T_CONST;
+  std::string constants;  // tape_body's arguments for them
+  for (unsigned k = 0; k < NC; ++k) constants += "constants.k[" + str(k) + "], ";
+
   std::string s = kMathSource;
+  if (NC) s += "\nstruct TapeConstants { float k[" + str(NC) + "]; };\n";
   s += "\n__device__ __forceinline__ void tape_body(";
+  for (unsigned k = 0; k < NC; ++k) s += "const float k" + str(k) + ", ";
   for (unsigned k = 0; k < NI; ++k) s += "const float " + v(k) + ", ";
   for (unsigned k = 0; k < NO; ++k) s += "float &r" + str(k) + (k + 1 < NO ? ", " : "");
   s += ") {\n";
-  for (unsigned t = 0; t < NT; ++t) s += "  const float " + v(NI + t) + " = " + expression(q.instr[t]) + ";\n";
+  for (unsigned t = 0, c = 0; t < NT; ++t) {
+    const bool constant = q.instr[t].op == VRHI_T_CONST;
+    s += "  const float " + v(NI + t) + " = " + expression(q.instr[t], "k" + str(c)) + ";";
+    if (constant && show_constants) {
+      uint32_t bits;
+      memcpy(&bits, &q.instr[t].imm, 4);
+      char buf[32];
+      snprintf(buf, sizeof buf, "  // 0x%08x", bits);
+      s += buf;
+    }
+    s += "\n";
+    c += constant;
+  }
   for (unsigned k = 0; k < NO; ++k) s += "  r" + str(k) + " = " + v(q.out_value[k]) + ";\n";
   s += "}\n\nextern \"C\" __global__ void __launch_bounds__(256) vrhi_tape_kernel(";
   for (unsigned k = 0; k < NI; ++k) s += "const float *__restrict__ in" + str(k) + ", ";
   for (unsigned k = 0; k < NO; ++k) s += "float *__restrict__ out" + str(k) + ", ";
+  if (NC) s += "const __grid_constant__ TapeConstants constants, ";
   s += "const " + ULL + " rows, const " + ULL + " groups, const unsigned int W, const unsigned int R, const unsigned int tail, const " + ULL + " cols, const " + ULL + " rem, const unsigned int fold) {\n";
   s += "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");  // a programmatic dependent of the kernel before it, and the next one of it\n  asm volatile(\"griddepcontrol.launch_dependents;\");\n";
   if (form == FLAT) {
@@ -263,7 +281,7 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
     std::string t = "      {\n";
     for (unsigned k = 0; k < NO; ++k) t += "        " + V + " o" + str(k) + ";\n";
     for (const std::string &c : comps) {
-      t += "        tape_body(";
+      t += "        tape_body(" + constants;
       for (unsigned k = 0; k < NI; ++k) {
         const std::string K = str(k);
         if (!used[k]) t += "0.0f, ";
@@ -305,7 +323,7 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
     for (unsigned j = 0; j < 4; ++j) {
       s += "    if (4ull * g + " + str(j) + "ull < rem) {\n      const " + ULL + " e = 4ull * i + " + str(j) + "ull;\n";
       for (unsigned k = 0; k < NO; ++k) s += "      float o" + str(k) + ";\n";
-      s += "      tape_body(";
+      s += "      tape_body(" + constants;
       for (unsigned k = 0; k < NI; ++k) {
         const std::string K = str(k);
         s += !used[k] ? std::string("0.0f") : shape(k) == 's' ? "s" + K : shape(k) == 'r' ? "x" + K + comps[j]
@@ -323,7 +341,7 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll) {
   if (form == FLAT) {  // the elements behind the last float4
     s += "  if (blockIdx.x == 0 && threadIdx.x < tail) {\n      const " + ULL + " e = 4ull * groups + threadIdx.x;\n";
     for (unsigned k = 0; k < NO; ++k) s += "      float o" + str(k) + ";\n";
-    s += "      tape_body(";
+    s += "      tape_body(" + constants;
     for (unsigned k = 0; k < NI; ++k) s += !used[k] ? std::string("0.0f, ") : shape(k) == 's' ? "s" + str(k) + ", " : "in" + str(k) + "[e], ";
     for (unsigned k = 0; k < NO; ++k) s += "o" + str(k) + (k + 1 < NO ? ", " : "");
     s += ");\n";
@@ -432,7 +450,10 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   int unroll = full_inputs >= 3 ? 1 : full_inputs == 2 ? 2 : 3;
   static const int env_unroll = env_int("VRHI_TAPE_UNROLL", 1, 8, 0), env_blocks = env_int("VRHI_TAPE_BLOCKS_PER_SM", 1, 32, 0);  // tuning aids
   if (env_unroll) unroll = env_unroll;
-  // cache key: everything the generated text depends on, as raw bytes (the text itself is only built on a miss)
+  // cache key: everything the generated text depends on, as raw bytes (the text itself is only built on a miss).  The values
+  // of constants are not among it.
+  struct { float k[VRHI_TAPE_MAX_INSTR]; } constants;
+  uint32_t n_constants = 0;
   std::string key;
   {
     const unsigned P = form == ROWS ? super_rows_of(q.cols) : 1u;
@@ -444,19 +465,20 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
       const vrhi_tape_instr &I = q.instr[t];
       const uint16_t f[4] = {I.op, I.a, I.b, I.c};
       key.append(reinterpret_cast<const char *>(f), sizeof f);
-      key.append(reinterpret_cast<const char *>(&I.imm), sizeof I.imm);
+      if (I.op == VRHI_T_CONST) constants.k[n_constants++] = I.imm;
     }
   }
   auto it = g_cache.find(key);
   if (it == g_cache.end()) {
-    const std::string src = generate(q, form, unroll);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     VRHI_CUDA(cudaStreamIsCapturing(st->s, &cap));
+    // a recording cannot wait for the compiler; what the interpreting kernel can do it does, with the same bits
+    if (cap != cudaStreamCaptureStatusNone && !(q.colsum_mask | q.total_mask)) return 1;
     if (cap != cudaStreamCaptureStatusNone)
       return fail(VRHI_ERR_INVALID, "this tape has not been compiled yet; run the operator once on the stream before recording it");
     VRHI_CUDA(cudaFree(nullptr));  // makes the device's primary context current for the driver calls below
     CUfunction fn = nullptr;
-    VRHI_TRY(compile(st->dev, src, &fn));
+    VRHI_TRY(compile(st->dev, generate(q, form, unroll), &fn));
     int resident = 0;
     if (g_driver.occupancy(&resident, fn, 256, 0) != CUDA_SUCCESS || resident < 1) resident = 4;
     it = g_cache.emplace(key, Compiled{fn, resident}).first;
@@ -489,7 +511,7 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
     if (gy > 65535) gy = 65535;
     if (gy == 0) gy = 1;
   }
-  void *args[VRHI_TAPE_MAX_INPUTS + VRHI_TAPE_MAX_OUTPUTS + 8];
+  void *args[VRHI_TAPE_MAX_INPUTS + VRHI_TAPE_MAX_OUTPUTS + 9];
   const float *in_copy[VRHI_TAPE_MAX_INPUTS];
   float *out_copy[VRHI_TAPE_MAX_OUTPUTS];
   int n_args = 0;
@@ -518,6 +540,7 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
     for (uint32_t k = 0; k < q.n_outputs; ++k) out_copy[k] = out[k];
   }
   for (uint32_t k = 0; k < q.n_outputs; ++k) args[n_args++] = &out_copy[k];
+  if (n_constants) args[n_args++] = &constants;
   args[n_args++] = &rows; args[n_args++] = &groups; args[n_args++] = &W; args[n_args++] = &R; args[n_args++] = &tail; args[n_args++] = &cols; args[n_args++] = &rem; args[n_args++] = &fold;
   CUlaunchAttribute attr{};
   attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
@@ -559,7 +582,7 @@ void tape_jit_counters(uint64_t *compiled, uint64_t *launches, int *compiler_ver
 
 // The generated source of a tape, for inspection and for tests that run without a GPU.
 std::string tape_jit_source(const vrhi_tape_params &q) {
-  return generate(q, form_of(q), 2);
+  return generate(q, form_of(q), 2, true);
 }
 
 }  // namespace vrhi
