@@ -346,6 +346,10 @@ struct Planner {
     P->total_mask |= (op == VRHI_R_MEAN_ALL ? 0x101u : 1u) << k;
   }
 
+  // Kernels that add up are compiled with the graph: a recording could not wait for that, and the graph may meet one before
+  // it has ever run (adding up a vector does not need scratch either, see tape_jit_launch).
+  int prepare_sums(const vrhi_tape_params &P) { return (P.colsum_mask | P.total_mask) ? tape_jit_prepare(g->dev, P) : VRHI_OK; }
+
   // Emit one map kernel computing `roots` (same shape, same stage).
   int emit_map(const std::vector<int> &roots, const std::set<int> &leaves, int st) {
     const int shape = g->nodes[roots[0]].shape;
@@ -441,6 +445,7 @@ struct Planner {
     } else {
       VRHI_TRY(op_id("map_tape", &s.op));
       s.params.assign((unsigned char *)&P, (unsigned char *)&P + sizeof P);
+      VRHI_TRY(prepare_sums(P));
       text << "map_tape    stage " << st << " shape=" << shape_name(shape) << " inputs=" << P.n_inputs << " outputs=" << P.n_outputs
            << " instr=" << P.n_instr;
       for (uint32_t k = 0; k < P.n_outputs; ++k)
@@ -664,9 +669,12 @@ struct Planner {
           s.order = next_order++;
           VRHI_TRY(vrhi_op_lookup("map_tape", &s.op));
           vrhi_tape_params P{};
-          P.size = sizeof P; P.n_inputs = 1; P.n_outputs = 1; P.rows = 1; P.cols = len;
+          P.size = sizeof P; P.n_inputs = 1; P.n_outputs = 1;
+          P.rows = in_shape == VRHI_SHAPE_ROWVEC ? 1 : g->rows;
+          P.cols = in_shape == VRHI_SHAPE_COLVEC ? 1 : g->cols;
           P.out_value[0] = 0;
           mark_total(&P, 0, n.op);
+          VRHI_TRY(prepare_sums(P));
           s.params.assign((unsigned char *)&P, (unsigned char *)&P + sizeof P);
           s.args = {flat_in, dst};
           s.text = "map_tape    stage " + std::to_string(st) + " n=" + std::to_string(len) + (n.op == VRHI_R_MEAN_ALL ? " (mean)" : " (flat sum)");

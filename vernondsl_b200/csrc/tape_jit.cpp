@@ -423,6 +423,57 @@ static bool jit_enabled() {
   return on;
 }
 
+// Rows in flight per thread: about three 16-byte loads (measured on B200 with the three-input chain, 6.8 TB/s).
+static int unroll_of(const vrhi_tape_params &q) {
+  static const int env_unroll = env_int("VRHI_TAPE_UNROLL", 1, 8, 0);  // tuning aid
+  if (env_unroll) return env_unroll;
+  int full_inputs = 0;
+  for (uint32_t k = 0; k < q.n_inputs; ++k)
+    if (!(((q.row_vector_mask | q.col_vector_mask | q.scalar_mask) >> k) & 1u)) ++full_inputs;
+  return full_inputs >= 3 ? 1 : full_inputs == 2 ? 2 : 3;
+}
+
+// The kernel of a tape, compiled if it is not there yet and the caller may wait for that; else 1.  g_mu is held.
+static int find_kernel(vrhi_device_t *dev, const vrhi_tape_params &q, bool may_compile, Compiled *out) {
+  const Form form = form_of(q);
+  const int unroll = unroll_of(q);
+  // cache key: everything the generated text depends on, as raw bytes (the text itself is only built on a miss).  The values
+  // of constants are not among it.
+  std::string key;
+  const unsigned P = form == ROWS ? super_rows_of(q.cols) : 1u;
+  const uint32_t head[12] = {(uint32_t)dev->ordinal, (uint32_t)unroll, (uint32_t)form, P, q.n_inputs, q.n_outputs, q.n_instr,
+                             q.row_vector_mask, q.col_vector_mask, q.scalar_mask, q.colsum_mask, q.total_mask};
+  key.append(reinterpret_cast<const char *>(head), sizeof head);
+  key.append(reinterpret_cast<const char *>(q.out_value), sizeof(uint32_t) * q.n_outputs);
+  for (uint32_t t = 0; t < q.n_instr; ++t) {  // field by field: padding bytes of the struct are not defined
+    const vrhi_tape_instr &I = q.instr[t];
+    const uint16_t f[4] = {I.op, I.a, I.b, I.c};
+    key.append(reinterpret_cast<const char *>(f), sizeof f);
+  }
+  auto it = g_cache.find(key);
+  if (it == g_cache.end()) {
+    if (!may_compile) return 1;
+    VRHI_CUDA(cudaFree(nullptr));  // makes the device's primary context current for the driver calls below
+    CUfunction fn = nullptr;
+    VRHI_TRY(compile(dev, generate(q, form, unroll), &fn));
+    int resident = 0;
+    if (g_driver.occupancy(&resident, fn, 256, 0) != CUDA_SUCCESS || resident < 1) resident = 4;
+    it = g_cache.emplace(key, Compiled{fn, resident}).first;
+    ++g_compiled;
+  }
+  *out = it->second;
+  return VRHI_OK;
+}
+
+int tape_jit_prepare(vrhi_device_t *dev, const vrhi_tape_params &q) {
+  VRHI_CUDA(cudaSetDevice(dev->ordinal));
+  std::lock_guard<std::mutex> lock(g_mu);
+  load_once();
+  if (!g_nvrtc.ok || !g_driver.ok) return VRHI_OK;
+  Compiled unused;
+  return find_kernel(dev, q, true, &unused);
+}
+
 // Returns VRHI_OK when the compiled kernel was launched, 1 when this tape or shape is left to the
 // interpreter (no NVRTC, switched off, unaligned pointers, a handful of elements), and an error code when
 // compilation or the launch failed.
@@ -441,51 +492,28 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   std::lock_guard<std::mutex> lock(g_mu);
   load_once();
   if (!g_nvrtc.ok || !g_driver.ok) return 1;
-  // About three 16-byte loads in flight per thread and six blocks per SM, all resident at once (one
-  // wave): measured on B200 with the three-input chain, 6.8 TB/s; eight blocks per SM spill into a second, partly
-  // filled wave and two rows per trip then cost 15 %.
-  int full_inputs = 0;
-  for (uint32_t k = 0; k < q.n_inputs; ++k)
-    if (!(((q.row_vector_mask | q.col_vector_mask | q.scalar_mask) >> k) & 1u)) ++full_inputs;
-  int unroll = full_inputs >= 3 ? 1 : full_inputs == 2 ? 2 : 3;
-  static const int env_unroll = env_int("VRHI_TAPE_UNROLL", 1, 8, 0), env_blocks = env_int("VRHI_TAPE_BLOCKS_PER_SM", 1, 32, 0);  // tuning aids
-  if (env_unroll) unroll = env_unroll;
-  // cache key: everything the generated text depends on, as raw bytes (the text itself is only built on a miss).  The values
-  // of constants are not among it.
-  struct { float k[VRHI_TAPE_MAX_INSTR]; } constants;
-  uint32_t n_constants = 0;
-  std::string key;
-  {
-    const unsigned P = form == ROWS ? super_rows_of(q.cols) : 1u;
-    const uint32_t head[12] = {(uint32_t)st->dev->ordinal, (uint32_t)unroll, (uint32_t)form, P, q.n_inputs, q.n_outputs, q.n_instr,
-                               q.row_vector_mask, q.col_vector_mask, q.scalar_mask, q.colsum_mask, q.total_mask};
-    key.append(reinterpret_cast<const char *>(head), sizeof head);
-    key.append(reinterpret_cast<const char *>(q.out_value), sizeof(uint32_t) * q.n_outputs);
-    for (uint32_t t = 0; t < q.n_instr; ++t) {  // field by field: padding bytes of the struct are not defined
-      const vrhi_tape_instr &I = q.instr[t];
-      const uint16_t f[4] = {I.op, I.a, I.b, I.c};
-      key.append(reinterpret_cast<const char *>(f), sizeof f);
-      if (I.op == VRHI_T_CONST) constants.k[n_constants++] = I.imm;
-    }
-  }
-  auto it = g_cache.find(key);
-  if (it == g_cache.end()) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  Compiled kernel;
+  int rc = find_kernel(st->dev, q, false, &kernel);
+  if (rc == 1) {
     VRHI_CUDA(cudaStreamIsCapturing(st->s, &cap));
     // a recording cannot wait for the compiler; what the interpreting kernel can do it does, with the same bits
     if (cap != cudaStreamCaptureStatusNone && !(q.colsum_mask | q.total_mask)) return 1;
     if (cap != cudaStreamCaptureStatusNone)
       return fail(VRHI_ERR_INVALID, "this tape has not been compiled yet; run the operator once on the stream before recording it");
-    VRHI_CUDA(cudaFree(nullptr));  // makes the device's primary context current for the driver calls below
-    CUfunction fn = nullptr;
-    VRHI_TRY(compile(st->dev, generate(q, form, unroll), &fn));
-    int resident = 0;
-    if (g_driver.occupancy(&resident, fn, 256, 0) != CUDA_SUCCESS || resident < 1) resident = 4;
-    it = g_cache.emplace(key, Compiled{fn, resident}).first;
-    ++g_compiled;
+    rc = find_kernel(st->dev, q, true, &kernel);
   }
+  if (rc != VRHI_OK) return rc;
+  struct { float k[VRHI_TAPE_MAX_INSTR]; } constants;
+  uint32_t n_constants = 0;
+  for (uint32_t t = 0; t < q.n_instr; ++t)
+    if (q.instr[t].op == VRHI_T_CONST) constants.k[n_constants++] = q.instr[t].imm;
+  // Six blocks per SM, all resident at once (one wave): measured on B200 with the three-input chain, eight blocks
+  // per SM spill into a second, partly filled wave and two rows per trip then cost 15 %.
+  static const int env_blocks = env_int("VRHI_TAPE_BLOCKS_PER_SM", 1, 32, 0);  // tuning aid
+  const int unroll = unroll_of(q);
   const int most_blocks = 6;
-  const uint64_t blocks_per_sm = env_blocks ? env_blocks : it->second.resident < most_blocks ? it->second.resident : most_blocks;
+  const uint64_t blocks_per_sm = env_blocks ? env_blocks : kernel.resident < most_blocks ? kernel.resident : most_blocks;
   const uint64_t target = (uint64_t)st->dev->prop.multiProcessorCount * blocks_per_sm;
   const unsigned P = form == ROWS ? super_rows_of(q.cols) : 1u;
   uint64_t rows = q.rows / P, groups, gx, gy = 1, cols = q.cols, rem = q.rows % P * q.cols;
@@ -517,7 +545,18 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   int n_args = 0;
   for (uint32_t k = 0; k < q.n_inputs; ++k) { in_copy[k] = in[k]; args[n_args++] = &in_copy[k]; }
   FinishJobs jobs{};
-  if (q.colsum_mask | q.total_mask) {
+  if (form == FLAT && q.total_mask && (q.rows == 1 || q.cols == 1) && !st->arena) {
+    // Sums of a vector on a stream without scratch.  A recording cannot allocate it: one block, as row_sum has for a vector,
+    // leaves its sum where the result goes.
+    VRHI_CUDA(cudaStreamIsCapturing(st->s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) gx = gy = 1;
+  }
+  if (q.total_mask && !q.colsum_mask && gx * gy == 1) {
+    for (uint32_t k = 0; k < q.n_outputs; ++k) {
+      out_copy[k] = out[k];
+      if (tape_total(q, k)) add_finish_job(&jobs, out[k], out[k], 1, 1, tape_mean(q, k) ? 1.0 / (double)n : 1.0);
+    }
+  } else if (q.colsum_mask | q.total_mask) {
     const size_t colsum_floats = (size_t)gy * P / fold * q.cols, total_floats = ((size_t)gx * gy + 3) & ~size_t(3);
     size_t floats = 0;
     for (uint32_t k = 0; k < q.n_outputs; ++k) floats += ((q.colsum_mask >> k) & 1u) ? (colsum_floats + 3) & ~size_t(3) : tape_total(q, k) ? total_floats : 0;
@@ -551,7 +590,7 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   cfg.hStream = reinterpret_cast<CUstream>(st->s);
   cfg.attrs = &attr;
   cfg.numAttrs = chains(st) ? 1 : 0;
-  CUresult cr = g_driver.launch_kernel(&cfg, it->second.fn, args, nullptr);
+  CUresult cr = g_driver.launch_kernel(&cfg, kernel.fn, args, nullptr);
   if (cr != CUDA_SUCCESS) {
     const char *msg = "?";
     g_driver.get_error_string(cr, &msg);

@@ -181,6 +181,7 @@ cudaError_t finish_partials(cudaStream_t s, const FinishJobs &jobs);
 // the interpreter) or an error code.
 int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *const *in, float *const *out);
 bool tape_jit_available();
+int tape_jit_prepare(vrhi_device_t *dev, const vrhi_tape_params &q);  // compiles the tape if it has not been
 void tape_jit_counters(uint64_t *compiled, uint64_t *launches, int *compiler_version, int *built_version);
 std::string tape_jit_source(const vrhi_tape_params &q);
 
