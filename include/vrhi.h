@@ -364,8 +364,7 @@ typedef struct vrhi_tape_params {
  * kernel: tapes that differ in nothing else share it. */
 #define VRHI_TAPE_FLAG_INTERPRET 1u
 #define VRHI_TAPE_FLAG_TOTALS 2u
-/* Tapes compiled so far in this process, launches of compiled tapes (those over rows of a multiple of 4
- * elements; the forms for other row lengths are not counted), the version of the run-time
+/* Tapes compiled so far in this process, launches of compiled tapes, the version of the run-time
  * compiler in use (major*1000 + minor*10; 0 before the first tape, or when there is none) and the
  * CUDA version the library was built with, counted the same way.  When the two versions are equal
  * the compiled and the interpreting kernel give the same bits; with another compiler version the

@@ -89,7 +89,8 @@ def chain_tape():
 
 def run_tape_both_ways(dev, stream, tape, inputs, out_shapes, rows, cols):
     """Runs the tape as a kernel compiled for it and through the interpreting kernel; the two must agree bit for
-    bit.  Where the compiled path applies (columns a multiple of 4) it must really have run."""
+    bit.  Where the compiled path applies (all but a few hundred elements in rows of no multiple of 4) it must
+    really have run."""
     outs_c = [dev.empty(s, np.float32) for s in out_shapes]
     outs_i = [dev.empty(s, np.float32) for s in out_shapes]
     before = ops.tape_jit_stats()["launches"]
@@ -98,7 +99,7 @@ def run_tape_both_ways(dev, stream, tape, inputs, out_shapes, rows, cols):
     ops.map_tape(stream, tape, inputs, outs_i, rows, cols, interpret=True)
     assert ops.tape_jit_stats()["launches"] - before == compiled_ran      # the flag really selects the interpreter
     stream.check()
-    assert compiled_ran == (1 if cols % 4 == 0 else 0)
+    assert compiled_ran == (1 if cols % 4 == 0 or rows * cols >= 256 else 0)
     got_c, got_i = [o.download() for o in outs_c], [o.download() for o in outs_i]
     info = ops.tape_jit_stats()
     for c, i in zip(got_c, got_i):

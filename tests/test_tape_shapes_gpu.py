@@ -1,5 +1,5 @@
-"""GPU: the three forms of a compiled tape (one long array with a tail, rows of float4 groups, rows of single
-elements) at the edges of their tiling, against the interpreting kernel (same bits) and, for summed
+"""GPU: the two forms of a compiled tape (one long array with a tail; rows, several at a time where their length is no
+multiple of 4) at the edges of their tiling, against the interpreting kernel (same bits) and, for summed
 outputs, binary64 sums of the stored values (1e-5 of the sum of magnitudes, as in test_rows_gpu.py)."""
 import numpy as np
 import pytest
@@ -34,8 +34,11 @@ def test_every_form_gives_the_interpreters_bits(dev, stream, rows, cols, broadca
     ref = [dev.empty((rows, cols), np.float32) for _ in range(2)]
     for b in got:
         b.fill(0xEE, stream=stream)
+    before = ops.tape_jit_stats()["launches"]
     ops.map_tape(stream, t, bufs, got, rows, cols)
+    assert ops.tape_jit_stats()["launches"] == before + 1      # not the interpreter against itself
     ops.map_tape(stream, t, bufs, ref, rows, cols, interpret=True)
+    assert ops.tape_jit_stats()["launches"] == before + 1
     stream.check()
     stored = [b.download() for b in ref]
     for g, r in zip(got, stored):

@@ -31,7 +31,10 @@ def test_the_interpreters_bits_and_the_sums(dev, stream):
             t, v = expression(**shapes)
             t.output(v)
             for o, interpret in zip(outs, (False, True)):
+                before = ops.tape_jit_stats()["launches"]
                 ops.map_tape(stream, t, ins, [o], rows, cols, interpret=interpret)
+                compiled = not interpret and rows * cols >= 256      # smaller ones are the interpreter's
+                assert ops.tape_jit_stats()["launches"] - before == compiled, (rows, cols)
             stream.check()
             got, want = (o.download() for o in outs)
             assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (rows, cols, shapes)
