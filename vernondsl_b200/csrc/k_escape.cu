@@ -91,6 +91,40 @@ static float escape_limit(uint32_t test, float bound) {
   return s;
 }
 
+// Steps from which the regrouping kernel is taken.  It pays about 2 us per tile and warp for intake and pool; the block
+// kernel runs a warp as long as its slowest pixel, and an image as long as the SM that drew the most such warps.  Which
+// costs more depends on how many tiles of 64 pixels a resident warp gets, hence on the pixels, and on the view.
+// Measured on B200, regrouping vs blocks in us, two or three views of each set (Julia: -0.8+0.156i, whose pixels all escape;
+// -0.123+0.745i, a fifth of whose pixels run to max_iter.  Mandelbrot: the whole set; -0.75+0.1i, 0.04 wide):
+//   Julia        256 steps               512                     1024                    2048
+//   128 x  64    7.3/7.1    7.3/7.0      10.9/12.5  11.2/12.4    15.7/19.6  19.4/23.2    15.5/19.6  35.3/44.7
+//   256 x 256    7.6/7.3    7.8/7.2      11.4/12.7  11.4/12.5    17.2/20.4  19.6/23.2    20.4/29.1  35.5/44.7
+//   360 x 360    11.9/7.5   12.0/7.6     18.5/12.7  19.0/12.7    26.0/22.4  34.5/23.5    26.3/29.3  64.0/45.0
+//   480 x 480    13.4/11.9  13.4/11.6    20.1/19.8  20.3/19.9    29.9/33.2  35.9/37.2    32.1/36.1  66.3/71.8
+//   560 x 560    14.1/13.7  14.8/13.8    20.8/21.1  23.6/24.7    31.1/32.4  42.3/46.3    34.2/34.7  79.0/89.7
+//   640 x 700    15.4/14.6  17.5/18.4    22.4/25.4  27.9/32.8    33.1/36.6  50.1/62.1    37.3/38.3  94.8/120.9
+//   720 x 720    17.0/18.4  19.2/16.8    24.0/32.0  30.4/29.5    34.3/47.9  55.9/55.6    37.7/48.4  104/107
+//   1920 x 1080  36.2/36.9  37.9/38.5    43.1/62.1  55.1/66.3    54.5/87.9  98.4/123.7   61.6/92.1  185/235  (192: 34.0/30.0 33.7/31.2)
+//   Mandelbrot
+//   128 x  64    8.1/7.1    8.1/6.3      11.9/12.7  12.2/10.8    21.1/23.7  20.9/19.8    38.6/46.2  38.0/37.5
+//   256 x 192    12.2/6.5   8.5/6.5      21.2/10.9  12.7/10.9    39.8/19.9  21.6/19.9    75.6/37.8  39.2/37.8
+//   400 x 400    13.6/11.1  19.0/14.9    22.8/19.1  30.7/27.0    42.4/35.6  55.7/48.9    82.1/68.2  101.7/89.8
+//   448 x 448    14.1/14.5  20.5/15.0    23.6/26.0  33.3/27.3    42.1/49.1  56.1/51.6    81.2/95.0  103.7/100.2
+//   640 x 320    13.9/12.5  20.0/15.1    23.0/21.4  31.8/27.1    43.0/38.8  55.5/51.5    79.9/73.7  99.3/100.4
+//   512 x 512    15.4/18.5  23.9/19.1    24.6/33.9  38.6/35.2    43.8/64.7  67.7/67.2    81.4/126   123/131
+//   720 x 720    20.5/19.3  35.5/29.3    30.6/35.2  55.4/52.3    50.5/63.7  95.5/96.8    93.0/120   171/178
+//   1024 x 768   23.7/26.5  46.0/39.7    35.1/46.5  72.4/69.4    58.7/87.2  126/127      104/166    220/234  (192: 20.6/21.6 38.9/31.9)
+// and 4096 x 4096, -0.8+0.156i / the whole set: 64 steps 107 vs 106 / 141 vs 127, 128 steps 130 vs 154 / 167 vs 188.
+// Where the views disagree the regrouping kernel is preferred: its time follows the number of steps, the block kernel's also
+// where in the image the long pixels lie.
+static uint32_t regroup_from(uint32_t kind, uint64_t pixels) {
+  constexpr uint32_t NEVER = 0xffffffffu;
+  constexpr uint64_t Ki = 1024;
+  if (pixels >= 4096 * Ki) return 96;
+  if (kind == VRHI_ESCAPE_MANDELBROT) return pixels < 24 * Ki ? 512 : pixels < 176 * Ki ? NEVER : pixels < 240 * Ki ? 1024 : pixels < 512 * Ki ? 512 : 192;
+  return pixels < 88 * Ki ? 512 : pixels < 144 * Ki ? NEVER : pixels < 288 * Ki ? 1024 : pixels < 448 * Ki ? 512 : 256;
+}
+
 int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const void *params, size_t params_size) {
   vrhi_escape_params q;
   VRHI_TRY(read_params(params, params_size, &q));
@@ -158,18 +192,10 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
   p.c2_unsafe_hi = 4.05f;
   const bool blocks_ok = p.limit >= 4.0f && p.limit < 3.0e38f && q.max_iter <= (1u << 30) &&
                          (q.kind == VRHI_ESCAPE_MANDELBROT || sqrt(c2) <= cmax) && !(q.flags & VRHI_ESCAPE_FLAG_CHECKED_ONLY);
-  // Two kernels with unchecked blocks.  The regrouping one (k_escape_pair.cu) pays about 2 us per tile and warp for intake
-  // and pool and then loses nothing to pixels that outlive their neighbours; the block kernel (k_escape_block.cu) runs a
-  // warp as long as its slowest pixel.  So regroup where pixels may run long and every warp sees many tiles.  Measured on B200,
-  // regrouping against blocks, Julia / Mandelbrot in us:
-  //   640 x 320     256 steps: 13.1 vs 10.9 / 15.2 vs 9.5       1024: 29.8 vs 31.3 / 49.6 vs 30.4
-  //   1920 x 1080   128: 31.1 vs 27.4 / 32.2 vs 30.4            256: 36.5 vs 43.3 / 39.9 vs 47.4     1024: 55 vs 103 / 83 vs 151
-  //   4096 x 4096   64: 107 vs 106 / 141 vs 127                 128: 130 vs 154 / 167 vs 188         256: 164 vs 251 / 212 vs 303
+  // Two kernels with unchecked blocks: the regrouping one (k_escape_pair.cu) loses nothing to pixels that outlive their
+  // neighbours, the block kernel (k_escape_block.cu) is cheaper per step and has no intake (see regroup_from).
   const uint64_t pixels = (uint64_t)q.width * p.rows_owned;
-  //   128 x 64      256: 7.2 vs 6.8 / 7.4 vs 7.0                1024: 14.9 vs 19.4 / 18.3 vs 23.6 (one tile per warp: the
-  //                 length of a warp's chain of blocks and votes is all there is)
-  const uint32_t regroup_from = pixels >= (4ull << 20) ? 96u : pixels >= (512ull << 10) ? 192u : pixels >= (64ull << 10) ? 0xffffffffu : 512u;
-  bool regroup_ok = blocks_ok && q.max_iter >= regroup_from && (uint64_t)q.width * q.height <= 0xffffffffull;
+  bool regroup_ok = blocks_ok && q.max_iter >= regroup_from(q.kind, pixels) && (uint64_t)q.width * q.height <= 0xffffffffull;
   // The regrouping kernel's work counter lives in the stream's scratch.  A launch of 64 steps or more with the a+b test asks
   // for it whichever kernel is chosen, so that recording one on a stream that has never run one is refused whatever the
   // image's size; any other launch is recorded there with the kernel that needs none.
