@@ -28,3 +28,28 @@ def test_both_sides_of_every_line(dev, stream, w, h, kind):
         assert np.array_equal(img.download(), ref.download()), max_iter
     for b in (img, ref):
         b.close()
+
+
+@pytest.mark.parametrize("max_iter", [600, 1200])
+def test_recorded_without_scratch(dev, max_iter):
+    """The regrouping kernel's work counter lives in the stream's scratch; a launch recorded on a stream that has none is
+    recorded with the block kernel."""
+    w, h = 700, 600
+    st = dev.stream()
+    dx, dy = ops.grid_steps(-2.0, 1.2, -1.2, 1.2, w, h)
+    img, ref = (dev.empty((h, w), np.uint32, L.IMAGE) for _ in range(2))
+    for kind in (L.JULIA, L.MANDELBROT):
+        p = ops.escape_params(kind, w, h, -2.0, -1.2, dx, dy, cr=-0.123, ci=0.745, max_iter=max_iter)
+        fresh = dev.stream()
+        img.fill(0xEE)
+        with fresh.record() as seq:
+            ops.escape_time(fresh, img, p)
+        assert seq.stats()["kernels"] == 1
+        seq.launch()
+        fresh.check()
+        ops.escape_time(st, ref, p)
+        st.check()
+        assert np.array_equal(img.download(), ref.download())
+        seq.close()
+        fresh.close()
+    st.close()

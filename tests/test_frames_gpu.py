@@ -112,16 +112,28 @@ def test_sequence_of_mixed_operators_matches_plain_launches():
 def test_recording_refuses_an_operator_whose_scratch_does_not_exist_yet():
     dev = vd.Device(0)
     st = dev.stream()                               # fresh stream: no scratch yet
-    img = dev.empty((64, 64), np.uint32, L.IMAGE)
-    p = ops.escape_params(L.MANDELBROT, 64, 64, -2.5, -1.0, 3.5 / 64, 2.0 / 64, max_iter=128)
+    rows, cols = 2000, 33                           # enough rows for several partial sums per column
+    m = np.random.default_rng(4).standard_normal((rows, cols)).astype(np.float32)
+    M, out = dev.from_numpy(m), dev.empty(cols, np.float32)
     with pytest.raises(vd.VrhiError) as err:
         with st.record():
-            ops.escape_time(st, img, p)
+            ops.col_sum(st, M, out, rows, cols)
     assert err.value.status == L.ERR_INVALID and "before recording" in str(err.value)
-    ops.escape_time(st, img, p)                     # the stream is usable afterwards
+    ops.col_sum(st, M, out, rows, cols)             # the stream is usable afterwards
     st.check()
+    assert np.abs(out.download() - m.astype(np.float64).sum(axis=0)).max() <= 1e-5 * np.abs(m).astype(np.float64).sum(axis=0).max()
+    # an image whose kernel needs no scratch is recorded on a stream that has none
+    fresh = dev.stream()
+    img = dev.empty((64, 64), np.uint32, L.IMAGE)
+    p = ops.escape_params(L.MANDELBROT, 64, 64, -2.5, -1.0, 3.5 / 64, 2.0 / 64, max_iter=128)
+    with fresh.record() as seq:
+        ops.escape_time(fresh, img, p)
+    seq.launch()
+    fresh.check()
     want, _ = oracle.escape_time(oracle.MANDELBROT, 64, 64, -2.5, -1.0, np.float32(3.5 / 64), np.float32(2.0 / 64), max_iter=128)
     assert np.array_equal(img.download(dtype=np.uint32, shape=(64, 64)), want)
+    seq.close()
+    fresh.close()
     st.close()
 
 
@@ -163,19 +175,18 @@ def test_a_recording_can_span_two_streams():
 
 
 def test_a_sequence_survives_the_growth_of_its_streams_scratch(dev, stream):
-    """A recorded sequence points into the stream's scratch of its time (the escape-time work counter
-    and the memset that clears it).  An operator that later needs more scratch than the stream holds
+    """A recorded sequence points into the stream's scratch of its time (the escape-time work counter).  An operator that later needs more scratch than the stream holds
     makes the stream allocate a larger block; the block the sequence points into must stay alive,
     and both the sequence and the operator must keep giving right answers."""
     W = H = 512
     dx, dy = ops.grid_steps(-1.6, 1.6, -1.6, 1.6, W, H)
-    p = ops.escape_params(L.JULIA, W, H, -1.6, -1.6, dx, dy, cr=-0.8, ci=0.156, max_iter=300)
+    p = ops.escape_params(L.JULIA, W, H, -1.6, -1.6, dx, dy, cr=-0.8, ci=0.156, max_iter=1100)   # regrouped
     img = dev.empty((H, W), np.uint32, L.IMAGE)
     ops.escape_time(stream, img, p)          # sizes the scratch (4 MiB at first use)
     stream.check()
     with stream.record() as seq:
         ops.escape_time(stream, img, p)
-    want, _ = oracle.escape_time(oracle.JULIA, W, H, -1.6, -1.6, dx, dy, -0.8, 0.156, 300)
+    want, _ = oracle.escape_time(oracle.JULIA, W, H, -1.6, -1.6, dx, dy, -0.8, 0.156, 1100)
     # column sums of [4096, 8192]: the partial rows need well over 4 MiB of scratch
     rows, cols = 4096, 8192
     m = np.random.default_rng(3).standard_normal((rows, cols)).astype(np.float32)

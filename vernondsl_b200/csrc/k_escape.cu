@@ -196,11 +196,8 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
   // neighbours, the block kernel (k_escape_block.cu) is cheaper per step and has no intake (see regroup_from).
   const uint64_t pixels = (uint64_t)q.width * p.rows_owned;
   bool regroup_ok = blocks_ok && q.max_iter >= regroup_from(q.kind, pixels) && (uint64_t)q.width * q.height <= 0xffffffffull;
-  // The regrouping kernel's work counter lives in the stream's scratch.  A launch of 64 steps or more with the a+b test asks
-  // for it whichever kernel is chosen, so that recording one on a stream that has never run one is refused whatever the
-  // image's size; any other launch is recorded there with the kernel that needs none.
-  const bool asks = blocks_ok && q.test == VRHI_TEST_NORM2_GT && q.max_iter >= 64u && (q.kind == VRHI_ESCAPE_MANDELBROT || c2 <= 2.25);
-  if (asks) VRHI_TRY(stream_arena(st, 0, nullptr, nullptr));
+  // The regrouping kernel's work counter lives in the stream's scratch.  A recording cannot allocate it, so on a stream that
+  // has none yet the block kernel is recorded.
   if (regroup_ok && !st->arena) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     VRHI_CUDA(cudaStreamIsCapturing(st->s, &cap));
