@@ -261,14 +261,18 @@ int launch_escape_time(vrhi_stream_t *st, const ArgView *args, int n_args, const
     // each warp then owns enough tiles to keep its pool busy and the drain at the end is shorter.
     uint64_t ctas = (nb + 7) / 8;
     const uint64_t px_total = (uint64_t)p.tiles_per_row * tile_px * p.rows_owned;
-    // Launches of less than 16 Mi pixels are usually one of several per step (a rank's rows
+    // Launches of less than 64 Mi pixels are usually one of several per step (a rank's rows
     // computed group by group, frames of a sequence): with 2 blocks per SM and no pinning the blocks of the next
     // launch move in beside the draining ones (measured, four launches of 1/32 of that image each on two streams:
     // 0.39 ms against 0.45 ms with 4 pinned blocks per SM).
     // Larger launches: 3 blocks per SM, pinned (measured on the 16384^2 image with 1024-pixel batches: 2.133 ms
-    // against 2.145 ms with 4; with 512-pixel batches 3, 4 and 5 gave 2.170, 2.164 and 2.165 ms; 4096 x 4096, 128 steps:
-    // Julia 129.6 us with 3, 136.5 with 2, Mandelbrot 182.8 and 190.9).
-    uint64_t per_sm = px_total < (16ull << 20) ? 2 : 3;
+    // against 2.145 ms with 4; with 512-pixel batches 3, 4 and 5 gave 2.170, 2.164 and 2.165 ms).
+    // Between 16 and 64 Mi pixels the third block pays on one stream while the steps are few, and always costs launches on
+    // two streams.  2 blocks / 3 pinned ones, us per launch on one stream and on two: 4096 x 4096, Julia, 256 steps 142/137
+    // and 123/134, 1024 steps 173/175 and 149/164; Mandelbrot, 256 steps 214/212 and 192/198, 6000 x 6000, 512 steps 560/566
+    // and 508/520.
+    const bool few_steps = px_total >= (16ull << 20) && q.max_iter < 512u;
+    uint64_t per_sm = px_total >= (64ull << 20) || few_steps ? 3 : 2;
     if (env_per_sm >= 1 && env_per_sm <= 6) per_sm = (uint64_t)env_per_sm;
     const uint64_t cap = (uint64_t)sms * per_sm;
     grid = (int)(ctas < cap ? ctas : cap);
