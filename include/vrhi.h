@@ -364,6 +364,9 @@ typedef struct vrhi_tape_params {
  * kernel: tapes that differ in nothing else share it. */
 #define VRHI_TAPE_FLAG_INTERPRET 1u
 #define VRHI_TAPE_FLAG_TOTALS 2u
+/* The tape's constants never change (the execution graph's do not): they are part of the compiled kernel,
+ * where the compiler can fold them, and another set of them is another kernel. */
+#define VRHI_TAPE_FLAG_LITERALS 4u
 /* Tapes compiled so far in this process, launches of compiled tapes, the version of the run-time
  * compiler in use (major*1000 + minor*10; 0 before the first tape, or when there is none) and the
  * CUDA version the library was built with, counted the same way.  When the two versions are equal

@@ -101,7 +101,7 @@ class TapeParams(C.Structure):
                 ("total_mask", C.c_uint32)]
 
 
-TAPE_FLAG_INTERPRET, TAPE_FLAG_TOTALS = 1, 2
+TAPE_FLAG_INTERPRET, TAPE_FLAG_TOTALS, TAPE_FLAG_LITERALS = 1, 2, 4
 
 
 class RowsParams(C.Structure):

@@ -12,8 +12,9 @@
 // the tape says so, and the transcendental primitives are the same functions (tape_math.cuh is
 // compiled into both).  The two paths therefore produce the same bits.
 //
-// The tape's constants are no part of the kernel: they are passed by value at each launch.  Two tapes that differ in nothing
-// else, such as the frames of a loop with a moving uniform, share one kernel.
+// The tape's constants are no part of the kernel unless the tape says that they never change (VRHI_TAPE_FLAG_LITERALS): they are
+// passed by value at each launch, so two tapes that differ in nothing else, such as the frames of a loop with a
+// moving uniform, share one kernel.
 //
 // NVRTC and the driver entry points are looked up at run time (dlopen, cudaGetDriverEntryPoint):
 // the library neither links against them nor needs them unless a tape is launched.  Where NVRTC is
@@ -130,6 +131,8 @@ void load_once() {
          drv("cuOccupancyMaxActiveBlocksPerMultiprocessor", &d.occupancy);
 }
 
+inline bool tape_literal(const vrhi_tape_params &q) { return (q.flags & VRHI_TAPE_FLAG_LITERALS) != 0; }
+
 std::string v(unsigned k) { return "v" + std::to_string(k); }
 
 // One SSA instruction as a C expression over the values v<k>; `constant` is the name of a constant's value.
@@ -208,8 +211,9 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll, bool show
   bool any_colsum = false, any_total = false;
   for (unsigned k = 0; k < NO; ++k) { any_colsum = any_colsum || colsum(k); any_total = any_total || total(k); }
 
+  const bool literal = tape_literal(q);
   unsigned NC = 0;
-  for (unsigned t = 0; t < NT; ++t) NC += q.instr[t].op == VRHI_T_CONST;
+  for (unsigned t = 0; t < NT; ++t) NC += q.instr[t].op == VRHI_T_CONST && !literal;
   std::string constants;  // tape_body's arguments for them
   for (unsigned k = 0; k < NC; ++k) constants += "constants.k[" + str(k) + "], ";
 
@@ -222,14 +226,13 @@ std::string generate(const vrhi_tape_params &q, Form form, int unroll, bool show
   s += ") {\n";
   for (unsigned t = 0, c = 0; t < NT; ++t) {
     const bool constant = q.instr[t].op == VRHI_T_CONST;
-    s += "  const float " + v(NI + t) + " = " + expression(q.instr[t], "k" + str(c)) + ";";
-    if (constant && show_constants) {
-      uint32_t bits;
-      memcpy(&bits, &q.instr[t].imm, 4);
-      char buf[32];
-      snprintf(buf, sizeof buf, "  // 0x%08x", bits);
-      s += buf;
-    }
+    uint32_t bits;
+    memcpy(&bits, &q.instr[t].imm, 4);
+    char value[48], comment[32];
+    snprintf(value, sizeof value, "__int_as_float((int)0x%08xu)", bits);
+    snprintf(comment, sizeof comment, "  // 0x%08x", bits);
+    s += "  const float " + v(NI + t) + " = " + expression(q.instr[t], literal ? value : "k" + str(c)) + ";";
+    if (constant && show_constants) s += comment;
     s += "\n";
     c += constant;
   }
@@ -438,17 +441,19 @@ static int find_kernel(vrhi_device_t *dev, const vrhi_tape_params &q, bool may_c
   const Form form = form_of(q);
   const int unroll = unroll_of(q);
   // cache key: everything the generated text depends on, as raw bytes (the text itself is only built on a miss).  The values
-  // of constants are not among it.
+  // of constants are among it only where the tape says so.
+  const bool literal = tape_literal(q);
   std::string key;
   const unsigned P = form == ROWS ? super_rows_of(q.cols) : 1u;
-  const uint32_t head[12] = {(uint32_t)dev->ordinal, (uint32_t)unroll, (uint32_t)form, P, q.n_inputs, q.n_outputs, q.n_instr,
-                             q.row_vector_mask, q.col_vector_mask, q.scalar_mask, q.colsum_mask, q.total_mask};
+  const uint32_t head[13] = {(uint32_t)dev->ordinal, (uint32_t)unroll, (uint32_t)form, P, q.n_inputs, q.n_outputs, q.n_instr,
+                             q.row_vector_mask, q.col_vector_mask, q.scalar_mask, q.colsum_mask, q.total_mask, literal};
   key.append(reinterpret_cast<const char *>(head), sizeof head);
   key.append(reinterpret_cast<const char *>(q.out_value), sizeof(uint32_t) * q.n_outputs);
   for (uint32_t t = 0; t < q.n_instr; ++t) {  // field by field: padding bytes of the struct are not defined
     const vrhi_tape_instr &I = q.instr[t];
     const uint16_t f[4] = {I.op, I.a, I.b, I.c};
     key.append(reinterpret_cast<const char *>(f), sizeof f);
+    if (literal) key.append(reinterpret_cast<const char *>(&I.imm), sizeof I.imm);
   }
   auto it = g_cache.find(key);
   if (it == g_cache.end()) {
@@ -507,7 +512,7 @@ int tape_jit_launch(vrhi_stream_t *st, const vrhi_tape_params &q, const float *c
   struct { float k[VRHI_TAPE_MAX_INSTR]; } constants;
   uint32_t n_constants = 0;
   for (uint32_t t = 0; t < q.n_instr; ++t)
-    if (q.instr[t].op == VRHI_T_CONST) constants.k[n_constants++] = q.instr[t].imm;
+    if (q.instr[t].op == VRHI_T_CONST && !tape_literal(q)) constants.k[n_constants++] = q.instr[t].imm;
   // Six blocks per SM, all resident at once (one wave): measured on B200 with the three-input chain, eight blocks
   // per SM spill into a second, partly filled wave and two rows per trip then cost 15 %.
   static const int env_blocks = env_int("VRHI_TAPE_BLOCKS_PER_SM", 1, 32, 0);  // tuning aid
