@@ -28,3 +28,37 @@ def test_col_sum_at_the_edges_of_its_tiles(dev, stream, rows, cols):
     assert np.array_equal(got[0], got[1])      # fixed order of additions
     M.close()
     c.close()
+
+
+def rows_per_thread(rows, cols, sms):
+    """How many rows a thread of the first stage adds, and how many threads of a block share a column (k_rows.cu, plan_col_sum)."""
+    vec = cols % 4 == 0
+    groups = cols // 4 if vec else cols
+    gx = -(-groups // (64 if vec else 128))
+    W = -(-groups // gx)
+    R = 256 // W
+    gy = max(1, min(sms * (5 if vec else 8) // gx, -(-rows // (8 * R)), 4096))
+    return -(-rows // (gy * R)), R
+
+
+@pytest.mark.parametrize("rows,cols", [(1024, 65535), (1024, 65536), (4096, 16384), (4097, 16381), (40000, 257), (33, 4)])
+def test_rounding_errors_do_not_add_up_along_the_rows(dev, stream, rows, cols):
+    """Every element is the same v, chosen so that one addition of v to a sum near the end of a thread's rows drops almost
+    half a unit, always to the same side: the error of a chain of n additions is then n/4 units of 2^-24, and only a
+    short chain stays inside the bound.  A thread adds whole groups of eight rows as trees (3 roundings, then one to the
+    running sum), or, single columns, into four running sums; the up to seven rows left over one by one; a block its R
+    sums as a tree.  The rest is binary64.  Equal values grow a running sum evenly: c additions to it lose (c + 1) / 2
+    units of the result at most, half the bound for arbitrary values."""
+    n, R = rows_per_thread(rows, cols, dev.sm_count)
+    unit = 2.0 ** (max(int(n - 1).bit_length(), 2) - 1 - 23)       # of sums in the upper half of a thread's range
+    v = np.float32(1 + int(0.49 * unit * 2 ** 23) * 2.0 ** -23)
+    m = np.full((rows, cols), v, np.float32)
+    M, c = dev.from_numpy(m), dev.empty(cols, np.float32)
+    ops.col_sum(stream, M, c, rows, cols)
+    stream.check()
+    chain = n // 8 if cols % 4 == 0 else n // 8 * 2
+    depth = (chain + 1) / 2 + 3 + n % 8 + int(R).bit_length() + 1
+    want = rows * float(v)
+    assert np.abs(c.download().astype(np.float64) - want).max() <= depth * 2.0 ** -24 * want, (n, R)
+    M.close()
+    c.close()

@@ -660,7 +660,7 @@ int launch_row_stats_softmax(vrhi_stream_t *st, const ArgView *args, int n_args,
 // Measured on B200 against one thread per column group and a block per row: [65536,4096] 166 -> 153 us
 // (7.0 TB/s), [4096,16385] 69 -> 48 us, [1000000,33] 463 -> 28 us, [1000,1001] 20.7 -> 5.0 us.
 constexpr int kColRowsInFlight = 8;
-template <bool VEC> constexpr int kColBlocksPerSm = VEC ? 5 : 8;  // 43 and 32 registers per thread
+template <bool VEC> constexpr int kColBlocksPerSm = VEC ? 5 : 8;  // 48 and 32 registers per thread
 
 template <bool VEC> struct ColValue { typedef float type; };
 template <> struct ColValue<true> { typedef float4 type; };
@@ -682,8 +682,10 @@ __global__ void __launch_bounds__(256, kColBlocksPerSm<VEC>) col_partial_kernel(
   const uint32_t sub = threadIdx.x / W, w = threadIdx.x - sub * W;
   const uint64_t g = (uint64_t)blockIdx.x * W + w;
   const bool active = sub < R && g < groups;
-  V acc;
+  V acc, sums[4];
   col_zero(acc);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) col_zero(sums[k]);
   if (active) {
     const uint64_t step = (uint64_t)gridDim.y * R;
     uint64_t r = (uint64_t)blockIdx.y * R + sub;
@@ -693,10 +695,28 @@ __global__ void __launch_bounds__(256, kColBlocksPerSm<VEC>) col_partial_kernel(
       V v[kColRowsInFlight];
 #pragma unroll
       for (int k = 0; k < kColRowsInFlight; ++k) v[k] = __ldcs(p + k * pstep);
+      // A wide matrix leaves few threads per column (four in [1024,65535]): rows added one by one would be a chain of 256
+      // roundings.  Groups of four columns are added as a tree per eight rows (32 + 3 roundings), single columns into four
+      // running sums (64 + 2), because their tree costs time ([4096,16385] 50.2 us, one by one and so 48.6; the running
+      // sums cost [1024,65535] 54.3 -> 55.9).  Relative error of that sum, values of mean 1: 1.2e-7 -> 5.1e-8.
+      if constexpr (VEC) {
 #pragma unroll
-      for (int k = 0; k < kColRowsInFlight; ++k) col_add(acc, v[k]);
+        for (int n = 1; n < kColRowsInFlight; n *= 2)
+#pragma unroll
+          for (int k = 0; k < kColRowsInFlight; k += 2 * n) col_add(v[k], v[k + n]);
+        col_add(acc, v[0]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kColRowsInFlight; ++k) col_add(sums[k & 3], v[k]);
+      }
     }
     for (; r < rows; r += step, p += pstep) col_add(acc, __ldcs(p));
+    if constexpr (!VEC) {
+      col_add(sums[0], sums[1]);
+      col_add(sums[2], sums[3]);
+      col_add(sums[0], sums[2]);
+      col_add(acc, sums[0]);
+    }
   }
   if (R > 1) {
     red[threadIdx.x] = acc;
