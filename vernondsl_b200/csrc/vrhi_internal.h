@@ -245,7 +245,10 @@ cudaError_t launch_dependent(Kern kern, dim3 grid, unsigned block, size_t dyn, c
 }
 // An operator's first kernel is chained to whatever came before it, but not in a recording: there the launches of the
 // other streams run beside it, and blocks that only wait would take their places (64 frames of 640 x 320 recorded on
-// two streams: 172 us, and 200 us chained).
+// two streams: 172 us, and 200 us chained).  Eager launches that go to two streams in turn do not suffer from it, us per
+// launch chained / not: 640 x 320 frames 5.0 / 6.7, 1080p Julia 22.9 / 23.7, softmax of [2048,2048] 4.3 / 4.9 and [8192,4096]
+// 38.7 / 38.7, column sums of [8192,4096] 23.0 / 23.4, gradients of [4096,4096] 54.7 / 55.3; on four streams the same but for
+// the last, 52.9 / 51.7.
 inline bool chains(const vrhi_stream_t *st) { return !st->recording; }
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;"); }
