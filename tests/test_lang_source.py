@@ -70,6 +70,8 @@ def g(): pass
 def h(): pass
 ''',
     "tabs": "def f(x):\n\tif x:\n\t\ty = 1\n\treturn x\nz = 2\n",
+    "a form feed in front of a line's indentation": "def f(x):\n    y = x\n\f    y = y + 1\n    return y\nz = 2\n",
+    "a form feed between functions": "def f(x):\n    return x\n\f\ndef g(): pass\n",
     "one line": "def f(x): return x\nz = 3\n",
     "else at the margin of if": """
 if True:

@@ -382,14 +382,17 @@ def _block(lines: List[str]) -> str:
     """The function that begins on the first line (its decorators included): everything up to the first line of code behind
     its ``def`` that is indented no deeper.  ``inspect.getblock`` finds the same end by tokenizing, which takes longer than
     parsing the block does.  A line inside a string, inside brackets or behind a backslash may stop the search too early;
-    what it then returns is no complete statement."""
-    margin = len(lines[0]) - len(lines[0].lstrip(" "))
+    what it then returns is no complete statement.  SyntaxError for indentation by anything but spaces."""
+    margin = len(lines[0]) - len(lines[0].lstrip())
     header, end = True, 0
     for k, line in enumerate(lines):
-        text = line.lstrip(" ")
-        if not text.strip() or text[0] == "#":
+        text = line.lstrip()
+        if not text or text[0] == "#":
             continue
-        if len(line) - len(text) <= margin:
+        indent = len(line) - len(text)
+        if line[:indent].strip(" "):
+            raise SyntaxError("indented by tabs or form feeds")
+        if indent <= margin:
             if not header:
                 break
             header = not text.startswith(("def ", "async "))
